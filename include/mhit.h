@@ -213,7 +213,7 @@ int mhit_device_state(mhit_handle* h, void** u, void** v, void** w, void** phi);
 /* Apply the pending mean removal to the resident u, v, w in place. */
 int mhit_sync_state(mhit_handle* h);
 
-/* Tile shapes of the stencil kernels: z chunk kz (a divisor of n; 0 = 32)
+/* Tile shapes of the stencil kernels: z chunk kz (a divisor of n; 0 = chosen by grid size)
  * and momentum tile height mty (8 or 16; 0 = the default for n).  Results do
  * not depend on them; the step graphs are re-captured on the next step. */
 int mhit_set_tiles(mhit_handle* h, int kz, int mty);

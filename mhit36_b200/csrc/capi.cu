@@ -883,7 +883,7 @@ int mhit_drop_count(mhit_handle* h, int capacity, int* ndrops, int64_t* cells, d
 }
 
 // Tile shapes of the stencil kernels: z chunk kz (a divisor of n, 0 =
-// default 32) and momentum tile height mty (8 or 16, 0 = default for n).
+// chosen by grid size) and momentum tile height mty (8 or 16, 0 = default for n).
 // Results do not depend on them; the step graphs are re-captured.
 int mhit_set_tiles(mhit_handle* h, int kz, int mty) {
   if (!h) return MHIT_ERR_INVALID;

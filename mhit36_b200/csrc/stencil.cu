@@ -25,10 +25,40 @@ namespace mhit {
 
 constexpr int TX = 32, TY = 8, NT = TX * TY;
 
-// Default z chunk of the stencil kernels: 64 planes from 512^3 up (measured
-// 2-3% faster than 32 there on B200; the grid still has >= 13 waves), 32
-// below, so that smaller grids keep enough CTAs.
-static int pick_kz(int n) { return n >= 512 ? 64 : (n >= 32 ? 32 : n); }
+// Default number of z chunks of a stencil kernel with `tiles` column tiles and
+// `slots` CTAs resident on the GPU.  Large grids: chunks of 32 planes, 64 from
+// 512^3 up (2-3% faster than 32 there; a chunk recomputes a few planes to
+// fill its rings).  A grid with less than two waves of such CTAs is split
+// further, to the number of chunks that gives the fewest iterations: an
+// iteration takes about the same time (2.4 us for FP64 phase) whether one or
+// two CTAs share an SM, so waves * (longest chunk + lead) is what counts, lead
+// being the planes a chunk recomputes.  Chunks need not divide n evenly.
+// B200, FP64 step against chunks of 32 planes everywhere (with project_kz):
+// 32^3 NS 108 -> 72 us a call, 64^3 182 -> 62 us a step, 128^3 277 -> 214,
+// 192^3 664 -> 627; chunks of 2 or 4 planes cost 128^3 30% and 256^3 30-80%.
+static int pick_chunks(int n, int tiles, int slots, int lead) {
+  const int nz = n / (n >= 512 ? 64 : 32);
+  if ((long long)tiles * nz >= 2LL * slots) return nz;
+  int best = nz;
+  long long cost = -1;
+  for (int q = nz; q <= n / 2; ++q) {
+    const long long waves = ((long long)tiles * q + slots - 1) / slots;
+    const long long c = waves * ((n + q - 1) / q + lead);
+    if (cost < 0 || c < cost) {
+      cost = c;
+      best = q;
+    }
+  }
+  return best;
+}
+// SMs of the current device.
+static int sm_count() {
+  int dev = 0, v = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess ||
+      cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || v < 1)
+    return 148;
+  return v;
+}
 
 // Momentum tile height.  Both tiles run 256 threads; the 16-row tile gives
 // each thread two rows.  Measured on B200 at 512^3: FP64 8 rows 3.06 ms,
@@ -208,7 +238,7 @@ __device__ __forceinline__ T inv_norm_plus(T s, T tiny) {
 // phimap: a __grid_constant__ parameter (single simulation), or a map in the
 // ensemble's slot table (gmaps: acquired through the tensor-map proxy first).
 template <class T, bool TMA>
-__device__ __forceinline__ void phase_body(const StencilArgs<T>& a, int KZ, int bx, int by, int bz,
+__device__ __forceinline__ void phase_body(const StencilArgs<T>& a, int nz, int bx, int by, int bz,
                                            const CUtensorMap* __restrict__ phimap, bool gmaps) {
   if (a.ctrl->status) return;
   constexpr int TY = PTY, NT = PNT;
@@ -242,7 +272,8 @@ __device__ __forceinline__ void phase_body(const StencilArgs<T>& a, int KZ, int 
   // and the log is skipped -- bitwise the same values.
   const T psi0 = eps * PsiMath<T>::log_ratio((T)0 + enumv, (T)1 - (T)0 + enumv, s_tab);
   const T psi1 = eps * PsiMath<T>::log_ratio((T)1 + enumv, (T)1 - (T)1 + enumv, s_tab);
-  const int x0 = bx * TX, y0 = by * TY, k0 = bz * KZ;
+  // z chunk bz of nz
+  const int x0 = bx * TX, y0 = by * TY, k0 = bz * n / nz, KZ = (bz + 1) * n / nz - k0;
   const int tid = threadIdx.x, tx = tid % TX, ty = tid / TX;
   constexpr int RY = TY / PPT;  // row step between a thread's output rows
   const int i = x0 + tx;
@@ -448,7 +479,7 @@ __device__ __forceinline__ void phase_body(const StencilArgs<T>& a, int KZ, int 
 // rhs_o; reads the NEW phi (the reference computes B4 after A7).
 // momentum tile height: 8 or 16 rows (a tuning choice per grid size)
 template <class T, bool PF, int MTYv, bool TMA>
-__device__ __forceinline__ void momentum_body(const StencilArgs<T>& a, int KZ, int bx, int by, int bz,
+__device__ __forceinline__ void momentum_body(const StencilArgs<T>& a, int nz, int bx, int by, int bz,
                                               const PlaneMaps* __restrict__ maps, bool gmaps) {
   if (a.ctrl->status) return;
   // MPT output rows per thread (rows ty + 8h): 256 threads for either tile
@@ -472,7 +503,8 @@ __device__ __forceinline__ void momentum_body(const StencilArgs<T>& a, int KZ, i
   const T f1 = (T)a.c.f1, f2 = (T)a.c.f2, f3 = (T)a.c.f3;
   const T alpha = (T)a.ctrl->alpha, beta = (T)a.ctrl->beta;
   const T mu = (T)a.ctrl->mean[0], mv = (T)a.ctrl->mean[1], mw = (T)a.ctrl->mean[2];
-  const int x0 = bx * TX, y0 = by * TY, k0 = bz * KZ;
+  // z chunk bz of nz
+  const int x0 = bx * TX, y0 = by * TY, k0 = bz * n / nz, KZ = (bz + 1) * n / nz - k0;
   const int tid = threadIdx.x, tx = tid % TX, ty = tid / TX;
   const int i = x0 + tx;
   const size_t nn = (size_t)n * n;
@@ -732,12 +764,15 @@ __device__ __forceinline__ void momentum_body(const StencilArgs<T>& a, int KZ, i
 // ============================================================ projection
 // C2 + R1 (multi/main.f90:873-903): u = ustar - dt/rho*(p - p_m)*dxi, with the
 // sums and maxima of the projected u, v, w reduced per CTA in FP64.
-// z planes per projection CTA: 64 where n allows, else 32 or 16 (512^3:
-// FP64 projection plus finalize 1.47 -> 1.41 ms against 16 planes, with a
-// quarter of the partials to reduce; FP32 projection 1.85 -> 1.49 ms).  The
-// FP64 loop takes it as a compile-time trip count (a run-time one measured
-// 1.79 ms there).
-__host__ __device__ constexpr int project_kz(int n) { return n % 64 == 0 ? 64 : (n % 32 == 0 ? 32 : 16); }
+// z planes per projection CTA: 64 where n allows (512^3: FP64 projection plus
+// finalize 1.47 -> 1.41 ms against 16 planes, with a quarter of the partials
+// to reduce; FP32 projection 1.85 -> 1.49 ms); fewer on small grids, so that
+// they too fill the GPU (FP64: 32^3 21 -> 8 us, 64^3 42 -> 9 us, 96^3 25 -> 14
+// us, 128^3 68 -> 30 us, 192^3 92 -> 86 us).  The FP64 loop takes it as a
+// compile-time trip count (a run-time one measured 1.79 ms at 512^3).
+__host__ __device__ constexpr int project_kz(int n) {
+  return n <= 96 ? 4 : (n <= 128 ? 8 : (n <= 192 ? 16 : (n % 64 == 0 ? 64 : 32)));
+}
 
 template <class T, int PKZ>
 __device__ __forceinline__ void project_body(const StencilArgs<T>& a, int bx, int by, int bz, int gx, int gy) {
@@ -1002,13 +1037,13 @@ __device__ __forceinline__ void finalize_body(const double* __restrict__ partial
 // Single simulation: block coordinates are the grid's.
 template <class T>
 __global__ void __launch_bounds__(PNT, phase_min_blocks<T>())
-    phase_kernel(StencilArgs<T> a, int KZ, const __grid_constant__ CUtensorMap phimap) {
-  phase_body<T, true>(a, KZ, blockIdx.x, blockIdx.y, blockIdx.z, &phimap, false);
+    phase_kernel(StencilArgs<T> a, const __grid_constant__ CUtensorMap phimap) {
+  phase_body<T, true>(a, gridDim.z, blockIdx.x, blockIdx.y, blockIdx.z, &phimap, false);
 }
 template <class T, bool PF, int MTYv>
 __global__ void __launch_bounds__(TX * 8, momentum_min_blocks<T>(PF, MTYv))
-    momentum_kernel(StencilArgs<T> a, int KZ, const __grid_constant__ PlaneMaps maps) {
-  momentum_body<T, PF, MTYv, true>(a, KZ, blockIdx.x, blockIdx.y, blockIdx.z, &maps, false);
+    momentum_kernel(StencilArgs<T> a, const __grid_constant__ PlaneMaps maps) {
+  momentum_body<T, PF, MTYv, true>(a, gridDim.z, blockIdx.x, blockIdx.y, blockIdx.z, &maps, false);
 }
 template <class T, int PKZ>
 __global__ void __launch_bounds__(NT, 4) project_kernel(StencilArgs<T> a) {
@@ -1026,25 +1061,23 @@ __global__ void __launch_bounds__(FNT) finalize_kernel(const double* __restrict_
 // covers the slots; each slot runs exactly the arithmetic of a single
 // simulation, so a result is the same alone and in any mix.
 template <class T>
-__global__ void __launch_bounds__(PNT, phase_min_blocks<T>()) phase_kernel_b(const SlotArgs<T>* __restrict__ slots, int KZ,
-                                                                            int zch) {
+__global__ void __launch_bounds__(PNT, phase_min_blocks<T>()) phase_kernel_b(const SlotArgs<T>* __restrict__ slots, int zch) {
   const int sl = blockIdx.z / zch;
   if (!slots[sl].active) return;
   StencilArgs<T> a = slots[sl].st;
   const int par = (int)(a.ctrl->nstep & 1);
   a.phi_in = slots[sl].phi[par];
   a.phi_out = slots[sl].phi[par ^ 1];
-  phase_body<T, true>(a, KZ, blockIdx.x, blockIdx.y, blockIdx.z - sl * zch, &slots[sl].maps.phase_phi[par], true);
+  phase_body<T, true>(a, zch, blockIdx.x, blockIdx.y, blockIdx.z - sl * zch, &slots[sl].maps.phase_phi[par], true);
 }
 template <class T, bool PF, int MTYv>
-__global__ void __launch_bounds__(TX * 8, momentum_min_blocks<T>(PF, MTYv)) momentum_kernel_b(const SlotArgs<T>* __restrict__ slots, int KZ,
-                                                                         int zch) {
+__global__ void __launch_bounds__(TX * 8, momentum_min_blocks<T>(PF, MTYv)) momentum_kernel_b(const SlotArgs<T>* __restrict__ slots, int zch) {
   const int sl = blockIdx.z / zch;
   if (!slots[sl].active) return;
   StencilArgs<T> a = slots[sl].st;
   const int par = (int)((a.ctrl->nstep + 1) & 1);
   if (PF) a.phi_in = slots[sl].phi[par];  // the updated phi
-  momentum_body<T, PF, MTYv, true>(a, KZ, blockIdx.x, blockIdx.y, blockIdx.z - sl * zch,
+  momentum_body<T, PF, MTYv, true>(a, zch, blockIdx.x, blockIdx.y, blockIdx.z - sl * zch,
                                    &slots[sl].maps.mom[MTYv == 16 ? 1 : 0][par], true);
 }
 template <class T, int PKZ>
@@ -1191,7 +1224,7 @@ template cudaError_t encode_slot_maps<double>(SlotArgs<double>*, int, bool);
 template cudaError_t encode_slot_maps<float>(SlotArgs<float>*, int, bool);
 
 int stencil_size_ok(int n) {
-  return n >= 32 && n % TX == 0 && n % TY == 0 && n % PTY == 0 && n % project_kz(n) == 0 && n % pick_kz(n) == 0;
+  return n >= 32 && n % TX == 0 && n % TY == 0 && n % PTY == 0 && n % project_kz(n) == 0;
 }
 
 int project_partials(int n) { return (n / TX) * (n / TY) * (n / project_kz(n)); }
@@ -1225,31 +1258,31 @@ cudaError_t prepare_stencils() {
 
 template <class T> cudaError_t launch_phase(const StencilArgs<T>& a, cudaStream_t st, int kz) {
   const int n = a.c.n;
-  if (kz <= 0) kz = pick_kz(n);
-  dim3 grid(n / TX, n / PTY, n / kz);
+  const int tiles = (n / TX) * (n / PTY);
+  dim3 grid(n / TX, n / PTY, kz > 0 ? n / kz : pick_chunks(n, tiles, phase_min_blocks<T>() * sm_count(), 4));
   CUtensorMap pm;
   cudaError_t e = plane_map(&pm, a.phi_in, n, PhaseGeo<T>::EX, PTY + 4);
   if (e) return e;
-  phase_kernel<T><<<grid, PNT, phase_smem<T>(), st>>>(a, kz, pm);
+  phase_kernel<T><<<grid, PNT, phase_smem<T>(), st>>>(a, pm);
   return cudaGetLastError();
 }
 
 template <class T> cudaError_t launch_momentum(const StencilArgs<T>& a, bool pf, cudaStream_t st, int kz, int mty) {
   const int n = a.c.n;
-  if (kz <= 0) kz = pick_kz(n);
   if (mty != 8) mty = 16;
-  dim3 grid(n / TX, n / mty, n / kz);
+  const int tiles = (n / TX) * (n / mty);
+  dim3 grid(n / TX, n / mty, kz > 0 ? n / kz : pick_chunks(n, tiles, momentum_min_blocks<T>(pf, mty) * sm_count(), 3));
   const size_t sm = momentum_smem<T>(pf, mty);
   PlaneMaps pm;
   memset(&pm, 0, sizeof(pm));
   cudaError_t e = mty == 8 ? momentum_maps<T, 8>(&pm, a, pf) : momentum_maps<T, 16>(&pm, a, pf);
   if (e) return e;
   if (mty == 8) {
-    if (pf) momentum_kernel<T, true, 8><<<grid, TX * 8, sm, st>>>(a, kz, pm);
-    else momentum_kernel<T, false, 8><<<grid, TX * 8, sm, st>>>(a, kz, pm);
+    if (pf) momentum_kernel<T, true, 8><<<grid, TX * 8, sm, st>>>(a, pm);
+    else momentum_kernel<T, false, 8><<<grid, TX * 8, sm, st>>>(a, pm);
   } else {
-    if (pf) momentum_kernel<T, true, 16><<<grid, TX * 8, sm, st>>>(a, kz, pm);
-    else momentum_kernel<T, false, 16><<<grid, TX * 8, sm, st>>>(a, kz, pm);
+    if (pf) momentum_kernel<T, true, 16><<<grid, TX * 8, sm, st>>>(a, pm);
+    else momentum_kernel<T, false, 16><<<grid, TX * 8, sm, st>>>(a, pm);
   }
   return cudaGetLastError();
 }
@@ -1260,7 +1293,9 @@ template <class T> cudaError_t launch_project(const StencilArgs<T>& a, cudaStrea
   switch (project_kz(n)) {
     case 64: project_kernel<T, 64><<<grid, NT, 0, st>>>(a); break;
     case 32: project_kernel<T, 32><<<grid, NT, 0, st>>>(a); break;
-    default: project_kernel<T, 16><<<grid, NT, 0, st>>>(a); break;
+    case 16: project_kernel<T, 16><<<grid, NT, 0, st>>>(a); break;
+    case 8: project_kernel<T, 8><<<grid, NT, 0, st>>>(a); break;
+    default: project_kernel<T, 4><<<grid, NT, 0, st>>>(a); break;
   }
   return cudaGetLastError();
 }
@@ -1297,7 +1332,7 @@ cudaError_t launch_wait_check(int arrive, long long limit_cycles, int* out_dev, 
 template <class T>
 cudaError_t launch_phase_batched(const SlotArgs<T>* slots, int nslots, int n, int kz, cudaStream_t st) {
   dim3 grid(n / TX, n / PTY, (n / kz) * nslots);
-  phase_kernel_b<T><<<grid, PNT, phase_smem<T>(), st>>>(slots, kz, n / kz);
+  phase_kernel_b<T><<<grid, PNT, phase_smem<T>(), st>>>(slots, n / kz);
   return cudaGetLastError();
 }
 template <class T>
@@ -1307,11 +1342,11 @@ cudaError_t launch_momentum_batched(const SlotArgs<T>* slots, int nslots, int n,
   dim3 grid(n / TX, n / mty, (n / kz) * nslots);
   const size_t sm = momentum_smem<T>(pf, mty);
   if (mty == 8) {
-    if (pf) momentum_kernel_b<T, true, 8><<<grid, TX * 8, sm, st>>>(slots, kz, n / kz);
-    else momentum_kernel_b<T, false, 8><<<grid, TX * 8, sm, st>>>(slots, kz, n / kz);
+    if (pf) momentum_kernel_b<T, true, 8><<<grid, TX * 8, sm, st>>>(slots, n / kz);
+    else momentum_kernel_b<T, false, 8><<<grid, TX * 8, sm, st>>>(slots, n / kz);
   } else {
-    if (pf) momentum_kernel_b<T, true, 16><<<grid, TX * 8, sm, st>>>(slots, kz, n / kz);
-    else momentum_kernel_b<T, false, 16><<<grid, TX * 8, sm, st>>>(slots, kz, n / kz);
+    if (pf) momentum_kernel_b<T, true, 16><<<grid, TX * 8, sm, st>>>(slots, n / kz);
+    else momentum_kernel_b<T, false, 16><<<grid, TX * 8, sm, st>>>(slots, n / kz);
   }
   return cudaGetLastError();
 }
@@ -1322,7 +1357,9 @@ cudaError_t launch_project_batched(const SlotArgs<T>* slots, int nslots, int n, 
     switch (project_kz(n)) {
       case 64: project_kernel_b<T, 64><<<grid, NT, 0, st>>>(slots, n / project_kz(n)); break;
       case 32: project_kernel_b<T, 32><<<grid, NT, 0, st>>>(slots, n / project_kz(n)); break;
-      default: project_kernel_b<T, 16><<<grid, NT, 0, st>>>(slots, n / project_kz(n)); break;
+      case 16: project_kernel_b<T, 16><<<grid, NT, 0, st>>>(slots, n / project_kz(n)); break;
+      case 8: project_kernel_b<T, 8><<<grid, NT, 0, st>>>(slots, n / project_kz(n)); break;
+      default: project_kernel_b<T, 4><<<grid, NT, 0, st>>>(slots, n / project_kz(n)); break;
     }
   } else
     project_refine_kernel_b<<<grid, NT, 0, st>>>(slots, n / project_kz(n));
