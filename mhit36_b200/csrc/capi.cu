@@ -68,6 +68,7 @@ struct mhit_handle {
   long long nstep_host = 0;
   bool has_fields = false;
   // drop counting scratch (allocated on first use)
+  unsigned* ccl_bits = nullptr;
   int* ccl_lab = nullptr;
   int* ccl_cnt = nullptr;
   int2* ccl_roots = nullptr;
@@ -848,8 +849,9 @@ int mhit_drop_count(mhit_handle* h, int capacity, int* ndrops, int64_t* cells, d
   DeviceGuard g(h->device);
   const int n = h->n;
   const size_t N3 = (size_t)n * n * n;
-  if (!h->ccl_lab) {
+  if (!h->ccl_counter) {
     h->ccl_cap = 1 << 20;
+    CK(h, dalloc(h, &h->ccl_bits, N3 / 8));
     CK(h, dalloc(h, &h->ccl_lab, N3 * sizeof(int)));
     CK(h, dalloc(h, &h->ccl_cnt, N3 * sizeof(int)));
     CK(h, dalloc(h, &h->ccl_roots, (size_t)h->ccl_cap * sizeof(int2)));
@@ -858,10 +860,10 @@ int mhit_drop_count(mhit_handle* h, int capacity, int* ndrops, int64_t* cells, d
   CK(h, pull_ctrl(h));
   const int cur = (int)(h->h_ctrl->nstep & 1);
   if (f32(h))
-    CK(h, mhit::launch_dropcount<float>(h->fphi[cur], n, h->ccl_lab, h->ccl_cnt, h->ccl_roots, h->ccl_cap,
+    CK(h, mhit::launch_dropcount<float>(h->fphi[cur], n, h->ccl_bits, h->ccl_lab, h->ccl_cnt, h->ccl_roots, h->ccl_cap,
                                         h->ccl_counter, h->st));
   else
-    CK(h, mhit::launch_dropcount<double>(h->phi[cur], n, h->ccl_lab, h->ccl_cnt, h->ccl_roots, h->ccl_cap,
+    CK(h, mhit::launch_dropcount<double>(h->phi[cur], n, h->ccl_bits, h->ccl_lab, h->ccl_cnt, h->ccl_roots, h->ccl_cap,
                                          h->ccl_counter, h->st));
   int cnt[2] = {0, 0};
   CK(h, cudaMemcpyAsync(cnt, h->ccl_counter, sizeof(cnt), cudaMemcpyDeviceToHost, h->st));

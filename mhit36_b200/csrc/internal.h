@@ -153,7 +153,7 @@ cudaError_t launch_stats(const T* u, const T* v, const T* w, const T* phi, const
 int stats_partials(int n);
 
 template <class T>
-cudaError_t launch_dropcount(const T* phi, int n, int* lab, int* cnt, int2* roots, int cap, int* d_counter,
-                             cudaStream_t st);
+cudaError_t launch_dropcount(const T* phi, int n, unsigned* bits, int* lab, int* cnt, int2* roots, int cap,
+                             int* d_counter, cudaStream_t st);
 
 }  // namespace mhit

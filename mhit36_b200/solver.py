@@ -149,12 +149,15 @@ class Solver:
         """Drop count and sizes of the current phi (post/DropCountSize convention):
         returns (cells, deq), numpy arrays in the reference's discovery order."""
         nd = ctypes.c_int()
-        self._check(self.lib.mhit_drop_count(self.h, 0, ctypes.byref(nd), None, None), "mhit_drop_count")
-        cells = np.empty(max(nd.value, 1), dtype=np.int64)
-        deq = np.empty(max(nd.value, 1))
-        self._check(self.lib.mhit_drop_count(self.h, nd.value, ctypes.byref(nd), cells.ctypes.data, deq.ctypes.data),
-                    "mhit_drop_count")
-        return cells[:nd.value], deq[:nd.value]
+        cap = 1024  # a count beyond it is taken again with room for all
+        while True:
+            cells = np.empty(cap, dtype=np.int64)
+            deq = np.empty(cap)
+            self._check(self.lib.mhit_drop_count(self.h, cap, ctypes.byref(nd), cells.ctypes.data, deq.ctypes.data),
+                        "mhit_drop_count")
+            if nd.value <= cap:
+                return cells[:nd.value], deq[:nd.value]
+            cap = nd.value
 
     # -- files
     def save(self, outdir: str, t: int):
