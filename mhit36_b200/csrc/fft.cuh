@@ -1,4 +1,4 @@
-// FFT building blocks of libmhit: radix-2/3/4/8 butterflies and the
+// FFT building blocks of libmhit: radix-2/3/4/8/12 butterflies and the
 // register-resident line transform (reg_fft_stages) that every x, y and z
 // pass of the Poisson solve uses.
 //
@@ -79,18 +79,49 @@ template <int DIR, class C> struct DFT<3, DIR, C> {
   }
 };
 
+// Good-Thomas: 12 = 3*4 with coprime factors, so with n = 4 n1 + 3 n2 and
+// k = 4 k1 + 9 k2 (mod 12) the transform is four DFTs of 3 and three of 4
+// with no twiddles between them.
+template <int DIR, class C> struct DFT<12, DIR, C> {
+  static __device__ __forceinline__ void run(C* v) {
+#pragma unroll
+    for (int n2 = 0; n2 < 4; ++n2) {
+      C u[3] = {v[(3 * n2) % 12], v[(4 + 3 * n2) % 12], v[(8 + 3 * n2) % 12]};
+      DFT<3, DIR, C>::run(u);
+#pragma unroll
+      for (int k1 = 0; k1 < 3; ++k1) v[(4 * k1 + 3 * n2) % 12] = u[k1];
+    }
+#pragma unroll
+    for (int k1 = 0; k1 < 3; ++k1) {
+      C a[4];
+#pragma unroll
+      for (int n2 = 0; n2 < 4; ++n2) a[n2] = v[(4 * k1 + 3 * n2) % 12];
+      dft4<DIR>(a[0], a[1], a[2], a[3]);
+#pragma unroll
+      for (int k2 = 0; k2 < 4; ++k2) v[(4 * k1 + 9 * k2) % 12] = a[k2];
+    }
+  }
+};
+
 // ---------------------------------------------------------------- register-resident lines
 // A line is spread over TPC = N/E threads, each holding E of its elements in
 // registers, v[m] = x[t + TPC*m] for thread t of the line: E = 8 for
 // power-of-two N, E = 12 for N = 3*2^k (96, 192, 384, 768).  Every stage's
-// radix R divides E (8, 4 or 2 for E = 8; 4, 2, 3 for E = 12, in that
-// order), and its butterflies run on registers -- butterfly b of the thread
-// is j = t + TPC*b with inputs v[b + (E/R)*r], which are x[j + r*N/R], the
+// radix R divides E (8, 4 or 2 for E = 8; 4, 2, 3 for E = 12, in that order,
+// or with R12 12, then 4 and 2), and its butterflies run on registers --
+// butterfly b of the thread is j = t + TPC*b with inputs v[b + (E/R)*r], which
+// are x[j + r*N/R], the
 // Stockham map of fft_stage -- and the data crosses shared memory only
 // between stages: a stage writes its outputs at their Stockham positions and
 // the next stage reads the canonical v[m] back.  The last stage's outputs are
 // the canonical positions themselves (NS*R = N makes them x[j + r*N/R]), so
 // they stay in registers.
+//
+// R12 takes one stage and one exchange out of the column passes, which are
+// bound by their shared-memory exchanges (384^3 FP64 on B200: z solve 388 ->
+// 346 us, y passes 223 -> 214; 192^3: 46 -> 41 and 31 -> 28).  The x passes go
+// without it: their lines follow one another in shared memory, and writes 12
+// elements apart conflict there (384^3: x inverse 225 -> 276 us).
 //
 // Exchange buffer: `at(n)` is the shared-memory slot of element n of the
 // thread's line.  The exchanges write either consecutive elements or
@@ -111,17 +142,18 @@ __device__ __forceinline__ int reg_pad(int n) { return n + (n >> 3); }
 __device__ __forceinline__ int reg_swz(int n) { return n ^ ((n >> 3) & 15); }
 // Elements per thread of a register-resident line of length N.
 __host__ __device__ constexpr int reg_elems(int N) { return (N & (N - 1)) == 0 ? 8 : 12; }
-constexpr int pick_radix_reg(int rem, int E) {
-  return (rem % 8 == 0 && E % 8 == 0) ? 8
+constexpr int pick_radix_reg(int rem, int E, bool r12) {
+  return (r12 && rem % 12 == 0 && E % 12 == 0) ? 12
+         : (rem % 8 == 0 && E % 8 == 0) ? 8
          : (rem % 4 == 0 && E % 4 == 0) ? 4
          : (rem % 2 == 0 && E % 2 == 0) ? 2
          : (rem % 3 == 0 && E % 3 == 0) ? 3 : rem;
 }
 
-template <int N, int NS, int DIR, class C, int E, class At>
+template <int N, int NS, int DIR, bool R12 = false, class C, int E, class At>
 __device__ __forceinline__ void reg_fft_stages(C (&v)[E], C* s, const C* __restrict__ tw, int t, const At& at) {
   if constexpr (NS < N) {
-    constexpr int R = pick_radix_reg(N / NS, E);
+    constexpr int R = pick_radix_reg(N / NS, E, R12);
     static_assert(E % R == 0 && (N / NS) % R == 0, "register-resident lines: the radix must divide E");
     constexpr int B = E / R, TPC = N / E, TSTRIDE = N / (NS * R);
 #pragma unroll
@@ -156,7 +188,7 @@ __device__ __forceinline__ void reg_fft_stages(C (&v)[E], C* s, const C* __restr
 #pragma unroll
       for (int m = 0; m < E; ++m) v[m] = s[at(t + TPC * m)];
       __syncthreads();
-      reg_fft_stages<N, NS * R, DIR, C, E>(v, s, tw, t, at);
+      reg_fft_stages<N, NS * R, DIR, R12>(v, s, tw, t, at);
     }
   }
 }

@@ -288,14 +288,14 @@ __device__ __forceinline__ void rcol_run(int total, const typename C2<T>::t* __r
     }
     C* col = static_cast<C*>(sl.spec) + c;
     if (KIND == 0) {
-      reg_fft_stages<N, 1, -1>(v, s, tw, t, at);
+      reg_fft_stages<N, 1, -1, true>(v, s, tw, t, at);
     } else if (KIND == 1) {
-      reg_fft_stages<N, 1, +1>(v, s, tw, t, at);
+      reg_fft_stages<N, 1, +1, true>(v, s, tw, t, at);
     } else {
       // forward z FFT, then -psi/k2/(nx*ny*nz) per mode (multi/main.f90:792,
       // one reciprocal per mode; mode (0,0,0) and the pitch padding beyond
       // kx = N/2 set to 0), then the inverse z FFT
-      reg_fft_stages<N, 1, -1>(v, s, tw, t, at);
+      reg_fft_stages<N, 1, -1, true>(v, s, tw, t, at);
       const double nnn = (double)((long long)N * (long long)N * (long long)N);
       const double* k2tab = sl.k2tab;
       const int mx = sl.m0 + c, jy = sl.jy;
@@ -313,7 +313,7 @@ __device__ __forceinline__ void rcol_run(int total, const typename C2<T>::t* __r
           v[m].y = v[m].y * f;
         }
       }
-      reg_fft_stages<N, 1, +1>(v, s, tw, t, at);
+      reg_fft_stages<N, 1, +1, true>(v, s, tw, t, at);
     }
 #pragma unroll
     for (int m = 0; m < E; ++m) col[(size_t)(t + TPC * m) * sl.stride] = v[m];
