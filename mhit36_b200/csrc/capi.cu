@@ -59,6 +59,7 @@ struct mhit_handle {
   // check) is recomputed on request.
   bool dp_in_spec = false;
   bool have_step = false;     // a step ran since the fields were set (ustar, p0 are its own)
+  double* stage = nullptr;    // FP32 form: device staging of FP64 planes for host copies (first use)
   double* div_out = nullptr;  // device: max |div u| of the FP64 projection (FP32 refine form)
   double* stat_partials = nullptr;
   double* stat_out = nullptr;
@@ -316,37 +317,49 @@ struct DevField {
   bool f32;
 };
 
-// host float64 (layout) -> device field; FP32 fields are rounded on the host.
+// FP32 fields cross the boundary through a device staging buffer of whole
+// FP64 planes (up to 32 MB, allocated on first use) and are rounded / widened
+// on the GPU: copy(chunk's first plane, planes) for each chunk, in stream order.
+template <class F> cudaError_t for_staged_planes(mhit_handle* h, const F& f) {
+  const int n = h->n;
+  const size_t plane = (size_t)n * n;
+  const int most = (int)std::min<size_t>(n, std::max<size_t>(1, ((size_t)4 << 20) / plane));
+  cudaError_t e;
+  if (!h->stage && (e = dalloc(h, &h->stage, plane * most * sizeof(double)))) return e;
+  for (int k = 0; k < n; k += most)
+    if ((e = f(k, std::min(most, n - k)))) return e;
+  return cudaSuccess;
+}
+
+// Host planes k .. k+planes-1 of a field in either layout, and their pitch.
+size_t host_offset(int n, int layout, int k) {
+  return layout == MHIT_LAYOUT_RAW ? (size_t)n * n * k : (size_t)n * (1 + (size_t)(n + 2) * (k + 1));
+}
+size_t host_pitch(int n, int layout) { return sizeof(double) * n * (size_t)(layout == MHIT_LAYOUT_RAW ? n : n + 2); }
+
+// host float64 (layout) -> device field.
 cudaError_t put_field(mhit_handle* h, DevField d, const double* src, int layout) {
   if (!d.f32) return upload(h, static_cast<double*>(d.ptr), src, layout);
   const int n = h->n;
-  const size_t plane = (size_t)n * n;
-  std::vector<float> tmp(plane * n);
-  for (int k = 0; k < n; ++k) {
-    const double* s = (layout == MHIT_LAYOUT_RAW) ? src + plane * k : src + (size_t)n * (1 + (size_t)(n + 2) * (k + 1));
-    float* t = tmp.data() + plane * k;
-    for (size_t q = 0; q < plane; ++q) t[q] = (float)s[q];
-  }
-  cudaError_t e = cudaMemcpyAsync(d.ptr, tmp.data(), tmp.size() * sizeof(float), cudaMemcpyHostToDevice, h->st);
-  if (e) return e;
-  return cudaStreamSynchronize(h->st);  // tmp dies here
+  const size_t plane = (size_t)n * n, pb = plane * sizeof(double);
+  return for_staged_planes(h, [&](int k, int planes) {
+    cudaError_t e = cudaMemcpy2DAsync(h->stage, pb, src + host_offset(n, layout, k), host_pitch(n, layout), pb, planes,
+                                      cudaMemcpyHostToDevice, h->st);
+    return e ? e : mhit::launch_narrow(h->stage, static_cast<float*>(d.ptr) + plane * k, plane * planes, h->st);
+  });
 }
 
-// device field -> host float64 (layout); synchronous for FP32 fields.
-cudaError_t get_field(mhit_handle* h, double* dst, DevField d, int layout) {
+// device field -> host float64 (layout); FP32 fields with `add`, if given, added in FP64.
+cudaError_t get_field(mhit_handle* h, double* dst, DevField d, int layout, const float* add = nullptr) {
   if (!d.f32) return download(h, dst, static_cast<const double*>(d.ptr), layout);
   const int n = h->n;
-  const size_t plane = (size_t)n * n;
-  std::vector<float> tmp(plane * n);
-  cudaError_t e = cudaMemcpyAsync(tmp.data(), d.ptr, tmp.size() * sizeof(float), cudaMemcpyDeviceToHost, h->st);
-  if (e) return e;
-  if ((e = cudaStreamSynchronize(h->st))) return e;
-  for (int k = 0; k < n; ++k) {
-    double* t = (layout == MHIT_LAYOUT_RAW) ? dst + plane * k : dst + (size_t)n * (1 + (size_t)(n + 2) * (k + 1));
-    const float* s = tmp.data() + plane * k;
-    for (size_t q = 0; q < plane; ++q) t[q] = (double)s[q];
-  }
-  return cudaSuccess;
+  const size_t plane = (size_t)n * n, pb = plane * sizeof(double);
+  return for_staged_planes(h, [&](int k, int planes) {
+    cudaError_t e = mhit::launch_widen(static_cast<const float*>(d.ptr) + plane * k, add ? add + plane * k : nullptr,
+                                       h->stage, plane * planes, h->st);
+    return e ? e : cudaMemcpy2DAsync(dst + host_offset(n, layout, k), host_pitch(n, layout), h->stage, pb, pb, planes,
+                                     cudaMemcpyDeviceToHost, h->st);
+  });
 }
 
 bool f32(mhit_handle* h) { return h->precision == MHIT_FP32_REFINE; }
@@ -711,22 +724,14 @@ int mhit_get_fields(mhit_handle* h, double* u, double* v, double* w, double* phi
   return MHIT_OK;
 }
 
-// The FP32 form's pressure is p0 + dp, summed in FP64 on the host.
+// The FP32 form's pressure is p0 + dp, summed in FP64.
 int mhit_get_pressure(mhit_handle* h, double* p, int layout) {
   if (!h || !p || !layout_ok(layout)) return MHIT_ERR_INVALID;
   DeviceGuard g(h->device);
   if (f32(h)) {
     CK(h, materialize_dp(h));
-    const size_t N3 = (size_t)h->n * h->n * h->n;
-    std::vector<double> a(N3), b(N3);
-    CK(h, get_field(h, a.data(), DevField{h->fp0, true}, MHIT_LAYOUT_RAW));
-    CK(h, get_field(h, b.data(), DevField{h->fdp, true}, MHIT_LAYOUT_RAW));
-    for (size_t q = 0; q < N3; ++q) a[q] += b[q];
-    const size_t plane = (size_t)h->n * h->n;
-    for (int k = 0; k < h->n; ++k) {
-      double* t = (layout == MHIT_LAYOUT_RAW) ? p + plane * k : p + (size_t)h->n * (1 + (size_t)(h->n + 2) * (k + 1));
-      memcpy(t, a.data() + plane * k, plane * sizeof(double));
-    }
+    CK(h, get_field(h, p, DevField{h->fp0, true}, layout, h->fdp));
+    CK(h, cudaStreamSynchronize(h->st));
   } else {
     if (h->p_in_spec) {  // the last step's pressure: x inverse of its spectrum
       mhit::PoissonArgs<double> pa;

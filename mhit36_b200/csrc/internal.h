@@ -152,6 +152,10 @@ cudaError_t launch_stats(const T* u, const T* v, const T* w, const T* phi, const
                          double dxi_d, double* partials, double* out, cudaStream_t st);
 int stats_partials(int n);
 
+// FP32 fields at the FP64 boundary: dst = (float)src; dst = a (+ b) in FP64.
+cudaError_t launch_narrow(const double* src, float* dst, size_t count, cudaStream_t st);
+cudaError_t launch_widen(const float* a, const float* b, double* dst, size_t count, cudaStream_t st);
+
 template <class T>
 cudaError_t launch_dropcount(const T* phi, int n, unsigned* bits, int* lab, int* cnt, int2* roots, int cap,
                              int* d_counter, cudaStream_t st);
