@@ -16,6 +16,7 @@
 #include <string>
 #include <vector>
 
+#include "hostcopy.h"
 #include "internal.h"
 #include "mhit.h"
 
@@ -59,6 +60,7 @@ struct mhit_handle {
   // check) is recomputed on request.
   bool dp_in_spec = false;
   bool have_step = false;     // a step ran since the fields were set (ustar, p0 are its own)
+  mhit::PinnedChunks chunks;  // for host copies of large pageable arrays (first use)
   double* stage = nullptr;    // FP32 form: device staging of FP64 planes for host copies (first use)
   double* div_out = nullptr;  // device: max |div u| of the FP64 projection (FP32 refine form)
   double* stat_partials = nullptr;
@@ -126,6 +128,7 @@ void free_all(mhit_handle* h) {
   h->allocs.clear();
   if (h->h_ctrl) cudaFreeHost(h->h_ctrl);
   if (h->h_stat) cudaFreeHost(h->h_stat);
+  h->chunks.release();
   if (h->st) cudaStreamDestroy(h->st);
 }
 
@@ -286,50 +289,11 @@ void reset_ctrl(mhit_handle* h) {
 
 int layout_ok(int layout) { return layout == MHIT_LAYOUT_RAW || layout == MHIT_LAYOUT_PIX_HALO; }
 
-// host (layout) -> device raw, n^2 doubles per z plane.
-cudaError_t upload(mhit_handle* h, double* dst, const double* src, int layout) {
-  const int n = h->n;
-  const size_t plane = (size_t)n * n;
-  if (layout == MHIT_LAYOUT_RAW) return cudaMemcpyAsync(dst, src, plane * n * sizeof(double), cudaMemcpyHostToDevice, h->st);
-  for (int k = 0; k < n; ++k) {
-    const double* s = src + (size_t)n * (1 + (size_t)(n + 2) * (k + 1));
-    cudaError_t e = cudaMemcpyAsync(dst + plane * k, s, plane * sizeof(double), cudaMemcpyHostToDevice, h->st);
-    if (e) return e;
-  }
-  return cudaSuccess;
-}
-
-cudaError_t download(mhit_handle* h, double* dst, const double* src, int layout) {
-  const int n = h->n;
-  const size_t plane = (size_t)n * n;
-  if (layout == MHIT_LAYOUT_RAW) return cudaMemcpyAsync(dst, src, plane * n * sizeof(double), cudaMemcpyDeviceToHost, h->st);
-  for (int k = 0; k < n; ++k) {
-    double* d = dst + (size_t)n * (1 + (size_t)(n + 2) * (k + 1));
-    cudaError_t e = cudaMemcpyAsync(d, src + plane * k, plane * sizeof(double), cudaMemcpyDeviceToHost, h->st);
-    if (e) return e;
-  }
-  return cudaSuccess;
-}
-
 // A device field of either form: FP64 or FP32 storage, raw layout.
 struct DevField {
   void* ptr;
   bool f32;
 };
-
-// FP32 fields cross the boundary through a device staging buffer of whole
-// FP64 planes (up to 32 MB, allocated on first use) and are rounded / widened
-// on the GPU: copy(chunk's first plane, planes) for each chunk, in stream order.
-template <class F> cudaError_t for_staged_planes(mhit_handle* h, const F& f) {
-  const int n = h->n;
-  const size_t plane = (size_t)n * n;
-  const int most = (int)std::min<size_t>(n, std::max<size_t>(1, ((size_t)4 << 20) / plane));
-  cudaError_t e;
-  if (!h->stage && (e = dalloc(h, &h->stage, plane * most * sizeof(double)))) return e;
-  for (int k = 0; k < n; k += most)
-    if ((e = f(k, std::min(most, n - k)))) return e;
-  return cudaSuccess;
-}
 
 // Host planes k .. k+planes-1 of a field in either layout, and their pitch.
 size_t host_offset(int n, int layout, int k) {
@@ -337,29 +301,79 @@ size_t host_offset(int n, int layout, int k) {
 }
 size_t host_pitch(int n, int layout) { return sizeof(double) * n * (size_t)(layout == MHIT_LAYOUT_RAW ? n : n + 2); }
 
+// A field crosses the boundary in chunks of whole planes (up to 16 MB of
+// float64), in stream order: f(first plane, planes).  FP32 fields pass
+// through a device buffer of one chunk, where they are rounded / widened.
+template <class F> cudaError_t for_chunks(mhit_handle* h, bool f32, const F& f) {
+  const int n = h->n;
+  const size_t pb = (size_t)n * n * sizeof(double);
+  const int most = (int)std::min<size_t>(n, std::max<size_t>(1, mhit::PinnedChunks::kBytes / pb));
+  cudaError_t e;
+  if (f32 && !h->stage && (e = dalloc(h, &h->stage, pb * most))) return e;
+  for (int k = 0; k < n; k += most)
+    if ((e = f(k, std::min(most, n - k)))) return e;
+  return cudaSuccess;
+}
+
 // host float64 (layout) -> device field.
 cudaError_t put_field(mhit_handle* h, DevField d, const double* src, int layout) {
-  if (!d.f32) return upload(h, static_cast<double*>(d.ptr), src, layout);
   const int n = h->n;
-  const size_t plane = (size_t)n * n, pb = plane * sizeof(double);
-  return for_staged_planes(h, [&](int k, int planes) {
-    cudaError_t e = cudaMemcpy2DAsync(h->stage, pb, src + host_offset(n, layout, k), host_pitch(n, layout), pb, planes,
-                                      cudaMemcpyHostToDevice, h->st);
-    return e ? e : mhit::launch_narrow(h->stage, static_cast<float*>(d.ptr) + plane * k, plane * planes, h->st);
+  const size_t plane = (size_t)n * n, pb = plane * sizeof(double), pitch = host_pitch(n, layout);
+  const bool chunks = mhit::wants_chunks(src, pb * n) && h->chunks.ready();
+  cudaError_t e;
+  int b = 0;
+  return for_chunks(h, d.f32, [&](int k, int planes) -> cudaError_t {
+    double* const to = d.f32 ? h->stage : static_cast<double*>(d.ptr) + plane * k;
+    const double* from = src + host_offset(n, layout, k);
+    size_t fp = pitch;
+    if (chunks) {
+      if ((e = cudaEventSynchronize(h->chunks.ev[b]))) return e;  // the chunk's previous copy has left it
+      mhit::parallel_copy(h->chunks.buf[b], pb, from, pitch, pb, planes);
+      from = static_cast<const double*>(h->chunks.buf[b]);
+      fp = pb;
+    }
+    if ((e = cudaMemcpy2DAsync(to, pb, from, fp, pb, planes, cudaMemcpyHostToDevice, h->st))) return e;
+    if (chunks && (e = cudaEventRecord(h->chunks.ev[b], h->st))) return e;
+    b ^= 1;
+    return d.f32 ? mhit::launch_narrow(h->stage, static_cast<float*>(d.ptr) + plane * k, plane * planes, h->st)
+                 : cudaSuccess;
   });
 }
 
 // device field -> host float64 (layout); FP32 fields with `add`, if given, added in FP64.
 cudaError_t get_field(mhit_handle* h, double* dst, DevField d, int layout, const float* add = nullptr) {
-  if (!d.f32) return download(h, dst, static_cast<const double*>(d.ptr), layout);
   const int n = h->n;
-  const size_t plane = (size_t)n * n, pb = plane * sizeof(double);
-  return for_staged_planes(h, [&](int k, int planes) {
-    cudaError_t e = mhit::launch_widen(static_cast<const float*>(d.ptr) + plane * k, add ? add + plane * k : nullptr,
-                                       h->stage, plane * planes, h->st);
-    return e ? e : cudaMemcpy2DAsync(dst + host_offset(n, layout, k), host_pitch(n, layout), h->stage, pb, pb, planes,
-                                     cudaMemcpyDeviceToHost, h->st);
+  const size_t plane = (size_t)n * n, pb = plane * sizeof(double), pitch = host_pitch(n, layout);
+  const bool chunks = mhit::wants_chunks(dst, pb * n) && h->chunks.ready();
+  cudaError_t e;
+  // the chunk on the link while the one before it is copied out
+  int b = 0, k_prev = 0, planes_prev = 0;
+  auto drain = [&]() -> cudaError_t {
+    if (!planes_prev) return cudaSuccess;
+    if ((e = cudaEventSynchronize(h->chunks.ev[b ^ 1]))) return e;
+    mhit::parallel_copy(dst + host_offset(n, layout, k_prev), pitch, h->chunks.buf[b ^ 1], pb, pb, planes_prev);
+    return cudaSuccess;
+  };
+  e = for_chunks(h, d.f32, [&](int k, int planes) -> cudaError_t {
+    const double* from = static_cast<const double*>(d.ptr) + plane * k;
+    if (d.f32) {
+      if ((e = mhit::launch_widen(static_cast<const float*>(d.ptr) + plane * k, add ? add + plane * k : nullptr,
+                                  h->stage, plane * planes, h->st)))
+        return e;
+      from = h->stage;
+    }
+    if (!chunks)
+      return cudaMemcpy2DAsync(dst + host_offset(n, layout, k), pitch, from, pb, pb, planes, cudaMemcpyDeviceToHost,
+                               h->st);
+    if ((e = cudaMemcpyAsync(h->chunks.buf[b], from, pb * planes, cudaMemcpyDeviceToHost, h->st))) return e;
+    if ((e = cudaEventRecord(h->chunks.ev[b], h->st))) return e;
+    if ((e = drain())) return e;
+    k_prev = k;
+    planes_prev = planes;
+    b ^= 1;
+    return cudaSuccess;
   });
+  return e ? e : (chunks ? drain() : cudaSuccess);
 }
 
 bool f32(mhit_handle* h) { return h->precision == MHIT_FP32_REFINE; }
@@ -743,7 +757,7 @@ int mhit_get_pressure(mhit_handle* h, double* p, int layout) {
       CK(h, mhit::launch_poisson_stage<double>(h->n, pa, 4, h->st));
       h->p_in_spec = false;
     }
-    CK(h, download(h, p, h->p, layout));
+    CK(h, get_field(h, p, DevField{h->p, false}, layout));
     CK(h, cudaStreamSynchronize(h->st));
   }
   if (layout == MHIT_LAYOUT_PIX_HALO) fill_halo_host(p, h->n);

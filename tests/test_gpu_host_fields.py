@@ -32,3 +32,19 @@ def test_round_trip(n, precision, layout):
         assert np.array_equal(y[core], want)
         if layout == capi.MHIT_LAYOUT_PIX_HALO:  # periodic halo
             assert np.array_equal(y[0], y[n]) and np.array_equal(y[:, n + 1], y[:, 1])
+
+
+@pytest.mark.parametrize("precision", ["fp64", "fp32"])
+def test_pinned_arrays(precision):
+    """Pinned arrays are copied without the staging chunks."""
+    import torch
+    from mhit36_b200 import Solver
+    from mhit36_b200.config import InputParams
+    n = 128
+    a = [torch.randn(n ** 3, dtype=torch.float64).pin_memory() for _ in range(4)]
+    got = [torch.zeros(n ** 3, dtype=torch.float64).pin_memory() for _ in range(4)]
+    with Solver(n, InputParams(k2_mode=1), precision=precision) as s:
+        s.set_fields_ptr(*[x.data_ptr() for x in a])
+        s.get_fields_ptr(*[x.data_ptr() for x in got])
+    for x, y in zip(a, got):
+        assert torch.equal(y, x.float().double() if precision == "fp32" else x)
