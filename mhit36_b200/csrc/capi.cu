@@ -49,7 +49,6 @@ struct mhit_handle {
   double* k2tab = nullptr;
   double *fsin = nullptr, *fcos = nullptr;
   double* partials = nullptr;
-  int nparts = 0;
   // FP64 step with the fused x inverse + projection: p is not stored by the
   // step; the spectrum still holds the last step's y-inverse output, from
   // which mhit_get_pressure recomputes p.
@@ -181,10 +180,10 @@ template <class T> mhit::StencilArgs<T> stencil_args(mhit_handle* h, int cur) {
 typedef std::pair<const char*, std::function<cudaError_t()>> Stage;
 
 // The kernels of one step reading phi[cur], in launch order.
-//   FP64: [phase] momentum xfwd yfwd zsolve yinv xinv project finalize
+//   FP64: [phase] momentum xfwd yfwd zsolve yinv xinv project
 //   FP32 refine: [phase] momentum, solve 1 (xfwd yfwd zsolve yinv xinv -> p0),
 //     solve 2 of the FP64 residual (xres yfwd2 zsolve2 yinv2 xinv2 -> dp),
-//     project (FP64), finalize
+//     project (FP64) [finalize]
 std::vector<Stage> step_stages(mhit_handle* h, int cur) {
   std::vector<Stage> v;
   cudaStream_t st = h->st;
@@ -212,11 +211,6 @@ std::vector<Stage> step_stages(mhit_handle* h, int cur) {
       v.push_back({"xinvproj", [pa, a, n, st] { return mhit::launch_xinv_project(n, pa, a, st); }});
     else
       v.push_back({"project", [a, st] { return mhit::launch_project<double>(a, st); }});
-    Ctrl* ctrl = h->ctrl;
-    double* part = h->partials;
-    int np = h->nparts;
-    StepConst c = h->c;
-    v.push_back({"finalize", [part, np, ctrl, c, st] { return mhit::launch_finalize(part, np, 6, ctrl, c, st); }});
   } else {
     mhit::StencilArgs<float> a = stencil_args<float>(h, cur);
     mhit::StencilArgs<float> am = a;
@@ -242,14 +236,6 @@ std::vector<Stage> step_stages(mhit_handle* h, int cur) {
       v.push_back({"xinvproj", [pr, a, n, st] { return mhit::launch_xinv_project<float>(n, pr, a, st); }});
     else
       v.push_back({"project", [a, dp, st] { return mhit::launch_project_refine(a, dp, st); }});
-    Ctrl* ctrl = h->ctrl;
-    double* part = h->partials;
-    int np = h->nparts;
-    StepConst c = h->c;
-    const int stride = fused ? 6 : 7;
-    v.push_back({"finalize", [part, np, ctrl, c, st, stride] {
-                   return mhit::launch_finalize(part, np, stride, ctrl, c, st);
-                 }});
   }
   return v;
 }
@@ -598,7 +584,6 @@ int mhit_create(const mhit_params* p, int nx, int ny, int nz, int precision, int
         break;
       }
     }
-    h->nparts = mhit::fused_projection(n) ? mhit::xinv_project_partials(n) : mhit::project_partials(n);
     if ((e = dalloc(h, &h->partials, (size_t)mhit::partials_capacity(n) * 7 * sizeof(double)))) {
       fail(e, "cudaMalloc partials");
       break;

@@ -18,7 +18,7 @@ struct Ctrl {
   double max_div;       // max |div u| of the FP64 projection (FP32 refine form)
   long long nstep;      // steps taken
   int status;           // sticky MHIT_* error; kernels return early when set
-  int pad_;
+  unsigned ticket;      // CTAs of the running projection that have finished (wraps to 0)
 };
 
 // Scalars fixed for the life of a handle, passed by value.

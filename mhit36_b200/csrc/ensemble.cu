@@ -609,12 +609,8 @@ cudaError_t enqueue_class_step(Class* c, int kz, int mty) {
     const bool fused = mhit::fused_projection(n) != 0;  // x inverse fused into the projection
     for (int k = 0; k < (fused ? 4 : 5); ++k)
       if ((err = mhit::launch_poisson_stage_batched<double>(t, S, n, k, 0, c->st))) return err;
-    if (fused) {
-      if ((err = mhit::launch_xinv_project_batched<double>(t, S, n, c->st))) return err;
-    } else if ((err = mhit::launch_project_batched<double>(t, S, n, c->st))) {
-      return err;
-    }
-    return mhit::launch_finalize_batched(t, S, n, c->st);
+    return fused ? mhit::launch_xinv_project_batched<double>(t, S, n, c->st)
+                 : mhit::launch_project_batched<double>(t, S, n, c->st);
   }
   const SlotArgs<float>* t = static_cast<const SlotArgs<float>*>(c->d_slots);
   if (c->pf && (err = mhit::launch_phase_batched<float>(t, S, n, kz, c->st))) return err;
@@ -625,12 +621,9 @@ cudaError_t enqueue_class_step(Class* c, int kz, int mty) {
   for (int w = 0; w < 2; ++w)
     for (int k = 0; k < ((w && fused) ? 4 : 5); ++k)
       if ((err = mhit::launch_poisson_stage_batched<float>(t, S, n, k, w, c->st))) return err;
-  if (fused) {
-    if ((err = mhit::launch_xinv_project_batched<float>(t, S, n, c->st))) return err;
-  } else if ((err = mhit::launch_project_batched<float>(t, S, n, c->st))) {
-    return err;
-  }
-  return mhit::launch_finalize_batched_f32(t, S, n, c->st);
+  if (fused) return mhit::launch_xinv_project_batched<float>(t, S, n, c->st);
+  if ((err = mhit::launch_project_batched<float>(t, S, n, c->st))) return err;
+  return mhit::launch_finalize_refine_batched(t, S, n, c->st);
 }
 
 cudaError_t capture_class(Class* c, int kz, int mty) {

@@ -92,8 +92,6 @@ template <class T>
 cudaError_t launch_momentum_batched(const SlotArgs<T>* slots, int nslots, int n, int kz, bool pf, cudaStream_t st,
                                    int mty);
 template <class T> cudaError_t launch_project_batched(const SlotArgs<T>* slots, int nslots, int n, cudaStream_t st);
-cudaError_t launch_finalize_batched(const SlotArgs<double>* slots, int nslots, int n, cudaStream_t st);
-cudaError_t launch_finalize_batched_f32(const SlotArgs<float>* slots, int nslots, int n, cudaStream_t st);
 // Poisson stage (0..4) for every slot; `which` 0 = po, 1 = pr.
 template <class T>
 cudaError_t launch_poisson_stage_batched(const SlotArgs<T>* slots, int nslots, int n, int stage, int which,
@@ -108,9 +106,8 @@ int default_mty(int n, int fp32);
 template <class T> cudaError_t launch_project(const StencilArgs<T>& a, cudaStream_t st);
 // FP32 refinement form: p = p0 + dp, projection and max|div u| in FP64.
 cudaError_t launch_project_refine(const StencilArgs<float>& a, const float* dp, cudaStream_t st);
-int project_refine_partials(int n);
-cudaError_t launch_finalize(const double* partials, int nparts, int stride, Ctrl* ctrl, StepConst c,
-                            cudaStream_t st);
+cudaError_t launch_finalize_refine(const StencilArgs<float>& a, cudaStream_t st);
+cudaError_t launch_finalize_refine_batched(const SlotArgs<float>* slots, int nslots, int n, cudaStream_t st);
 template <class T> cudaError_t launch_materialize(T* u, T* v, T* w, int n, Ctrl* ctrl, cudaStream_t st);
 cudaError_t prepare_stencils();
 int project_partials(int n);
@@ -140,9 +137,7 @@ template <class T> cudaError_t encode_column_maps(SlotMaps* m, const void* spec,
 // One-warp self-check of the bounded barrier wait (writes 0 or MHIT_ERR_TIMEOUT).
 cudaError_t launch_wait_check(int arrive, long long limit_cycles, int* out_dev, cudaStream_t st);
 cudaError_t launch_refine_divergence(const StencilArgs<float>& a, const float* dp, double* out, cudaStream_t st);
-// Partials the FP64 step's projection writes, and the buffer size that
-// holds either projection's partials (stride 7).
-inline int step_partials_fp64(int n) { return fused_projection(n) ? xinv_project_partials(n) : project_partials(n); }
+// Buffer size that holds either projection's partials (stride 7).
 inline int partials_capacity(int n) {
   return project_partials(n) > xinv_project_partials(n) ? project_partials(n) : xinv_project_partials(n);
 }

@@ -20,6 +20,7 @@
 #include <algorithm>
 #include "common.cuh"
 #include "fft.cuh"
+#include "finish.cuh"
 #include <string.h>
 #include "internal.h"
 
@@ -691,6 +692,7 @@ __device__ __forceinline__ void xinvproj_body(const typename C2<T>::t* __restric
     const size_t b = (size_t)bx + (size_t)gx * bz;
     for (int c = 0; c < 6; ++c) a.partials[b * 6 + c] = r6[c];
   }
+  finish_step<NT, 6>(a.partials, X::PARTS, a.ctrl, a.c);
 }
 
 template <int N, class T>
