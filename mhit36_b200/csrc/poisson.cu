@@ -611,43 +611,48 @@ __device__ __forceinline__ void xinvproj_body(const typename C2<T>::t* __restric
         }
       }
     }
-    __syncthreads();
     // (3) projection of plane kw (the chunk's first pass only fills spp).
-    // A thread's points are tid + NT*it; they are taken in groups of PG
-    // whose ustar/vstar/wstar loads are all issued before the group's
-    // arithmetic and stores (ustar and u are distinct arrays), so that a
-    // group costs one memory latency rather than PG.
+    // A thread's points are tid + NT*it, taken in groups of PG.  The first
+    // group's ustar/vstar/wstar loads are issued before the barrier and each
+    // further group's before the arithmetic of the one ahead of it (ustar and
+    // u are distinct arrays), so that a plane waits for memory about once
+    // (512^3 on B200: FP64 1541 -> 1384 us, FP32 1116 -> 968 us).
     if (kk >= k0) {
-#pragma unroll 1
-      for (int it0 = 0; it0 < PIT; it0 += PG) {
-        T lu[PG], lv[PG], lw[PG];
+      constexpr int NG = (PIT + PG - 1) / PG;
+      T lu[2][PG], lv[2][PG], lw[2][PG];
+      const size_t gk = (size_t)N * j0 + nn * kw;  // the plane's rows are contiguous: point pi is at gk + pi
+      const auto load = [&](int b, int it0) {
 #pragma unroll
         for (int c = 0; c < PG; ++c) {
           const int pi = threadIdx.x + NT * (it0 + c);
-          if (pi < 2 * P * N) {
-            const int x = pi % N, r = pi / N;
-            const size_t g = (size_t)x + (size_t)N * (j0 + r) + nn * kw;
-            lu[c] = us[g];
-            lv[c] = vs[g];
-            lw[c] = ws[g];
+          if (it0 + c < PIT && pi < 2 * P * N) {
+            lu[b][c] = us[gk + pi];
+            lv[b][c] = vs[gk + pi];
+            lw[b][c] = ws[gk + pi];
           }
         }
+      };
+      load(0, 0);
+      __syncthreads();
+#pragma unroll
+      for (int gr = 0; gr < NG; ++gr) {
+        const int it0 = gr * PG, b = gr & 1;
+        if (gr + 1 < NG) load(b ^ 1, it0 + PG);
 #pragma unroll
         for (int c = 0; c < PG; ++c) {
           const int pi = threadIdx.x + NT * (it0 + c);
-          if (pi < 2 * P * N) {
+          if (it0 + c < PIT && pi < 2 * P * N) {
             const int x = pi % N, r = pi / N;
-            const double pc = sp[(r + 1) * N + x];
+            const double pc = sp[N + pi];
             const double pxm = sp[(r + 1) * N + (x ? x - 1 : N - 1)];
-            const double pym = sp[r * N + x];
-            const double pzm = spp[r * N + x];
-            const size_t g = (size_t)x + (size_t)N * (j0 + r) + nn * kw;
-            const double uo = (double)lu[c] - dtr * (pc - pxm) * dxi;
-            const double vo = (double)lv[c] - dtr * (pc - pym) * dxi;
-            const double wo = (double)lw[c] - dtr * (pc - pzm) * dxi;
-            uo_[g] = (T)uo;
-            vo_[g] = (T)vo;
-            wo_[g] = (T)wo;
+            const double pym = sp[pi];
+            const double pzm = spp[pi];
+            const double uo = (double)lu[b][c] - dtr * (pc - pxm) * dxi;
+            const double vo = (double)lv[b][c] - dtr * (pc - pym) * dxi;
+            const double wo = (double)lw[b][c] - dtr * (pc - pzm) * dxi;
+            uo_[gk + pi] = (T)uo;
+            vo_[gk + pi] = (T)vo;
+            wo_[gk + pi] = (T)wo;
             su += uo;
             sv += vo;
             sw += wo;
@@ -656,11 +661,12 @@ __device__ __forceinline__ void xinvproj_body(const typename C2<T>::t* __restric
             xw = fmax(xw, wo);
             // NaN must not vanish in fmax: fold it into the sums too
             if (uo != uo || vo != vo || wo != wo) su = NAN;
-            spp[r * N + x] = pc;
+            spp[pi] = pc;
           }
         }
       }
     } else {
+      __syncthreads();
       for (int pi = threadIdx.x; pi < 2 * P * N; pi += NT) spp[pi] = sp[N + pi];
     }
     __syncthreads();  // sp (which aliases sx) is free for the next transform
