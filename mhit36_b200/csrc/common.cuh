@@ -83,17 +83,21 @@ __device__ __forceinline__ void mbar_arrive(unsigned long long* b) {
 // Wait for the phase with the given parity to complete, giving up once
 // `limit_cycles` SM clock cycles have passed (a poll may suspend the thread
 // for a short hardware time limit).  Returns false if it gave up.
+__device__ __forceinline__ bool mbar_try(unsigned a, unsigned parity) {
+  unsigned done;
+  asm volatile(
+      "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}\n"
+      : "=r"(done)
+      : "r"(a), "r"(parity)
+      : "memory");
+  return done != 0;
+}
 __device__ __forceinline__ bool mbar_wait(unsigned long long* b, unsigned parity, long long limit_cycles) {
   const unsigned a = smem_addr(b);
+  if (mbar_try(a, parity)) return true;
   const long long t0 = clock64();
   for (;;) {
-    unsigned done;
-    asm volatile(
-        "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}\n"
-        : "=r"(done)
-        : "r"(a), "r"(parity)
-        : "memory");
-    if (done) return true;
+    if (mbar_try(a, parity)) return true;
     if (clock64() - t0 > limit_cycles) return false;
   }
 }

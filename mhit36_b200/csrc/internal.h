@@ -61,14 +61,18 @@ template <class T> struct StencilArgs {
 struct PlaneMaps {
   CUtensorMap u, v, w, phi;
 };
+// Tensor maps of the phase kernel's staged planes.
+struct PhaseMaps {
+  CUtensorMap phi, u, v, w;
+};
 // Tensor maps of a served-ensemble slot, kept in its device table entry:
 // the momentum kernel's boxes per tile height (8, 16) and phi parity, the
-// phase kernel's phi box per parity, and the column passes' spectrum views
+// phase kernel's boxes per parity, and the column passes' spectrum views
 // (y passes, z solve).  Written by a kernel, so readers acquire them through
 // the tensor-map proxy before use.
 struct SlotMaps {
   PlaneMaps mom[2][2];
-  CUtensorMap phase_phi[2];
+  PhaseMaps phase[2];
   CUtensorMap col_y, col_z;
 };
 

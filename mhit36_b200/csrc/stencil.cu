@@ -31,9 +31,9 @@ constexpr int TX = 32, TY = 8, NT = TX * TY;
 // 512^3 up (2-3% faster than 32 there; a chunk recomputes a few planes to
 // fill its rings).  A grid with less than two waves of such CTAs is split
 // further, to the number of chunks that gives the fewest iterations: an
-// iteration takes about the same time (2.4 us for FP64 phase) whether one or
-// two CTAs share an SM, so waves * (longest chunk + lead) is what counts, lead
-// being the planes a chunk recomputes.  Chunks need not divide n evenly.
+// iteration takes about the same time (2.4 us for FP64 phase) however many CTAs
+// share an SM, so waves * (longest chunk + lead) is what counts, lead being the
+// planes a chunk recomputes.  Chunks need not divide n evenly.
 // B200, FP64 step against chunks of 32 planes everywhere (with project_kz):
 // 32^3 NS 108 -> 72 us a call, 64^3 182 -> 62 us a step, 128^3 277 -> 214,
 // 192^3 664 -> 627; chunks of 2 or 4 planes cost 128^3 30% and 256^3 30-80%.
@@ -96,21 +96,23 @@ __device__ __forceinline__ double div_nr(double a, double b) {
   return fma(fma(-b, q, a), y, q);
 }
 
-// log x for positive normal x; tab = g_log_table (in shared memory)
+// log x for positive normal x; tab = g_log_table (in shared memory).  The
+// integers k and j become doubles by their bit patterns (2^52 + k, and F
+// itself) instead of conversion instructions.
 __device__ __forceinline__ double tang_log(double x, const double* __restrict__ tab) {
   const int hi = __double2hiint(x), lo = __double2loint(x);
-  const int k = (hi >> 20) - 1023;
   const int mant = hi & 0x000fffff;
   const int j = (mant + (1 << 12)) >> 13;  // nearest j/128, 0..128
   const double m = __hiloint2double(mant | 0x3ff00000, lo);
-  const double r = (m - (1.0 + (double)j * (1.0 / 128))) * tab[j];  // m - F is exact
+  const double F = __hiloint2double(0x3ff00000 + (j << 13), 0);
+  const double kd = __hiloint2double(0x43300000, hi >> 20) - (4503599627370496.0 + 1023.0);
+  const double r = (m - F) * tab[j];  // m - F is exact
   double p = fma(r, 1.0 / 7, -1.0 / 6);
   p = fma(p, r, 0.2);
   p = fma(p, r, -0.25);
   p = fma(p, r, 1.0 / 3);
   p = fma(p, r, -0.5);
   p = fma(p, r * r, r);
-  const double kd = (double)k;
   return fma(kd, tab[3 * 129], tab[129 + j]) + (fma(kd, tab[3 * 129 + 1], tab[2 * 129 + j]) + p);
 }
 
@@ -165,9 +167,9 @@ static cudaError_t upload_log_table() {
 constexpr int PTY = 16;            // phase tile height
 constexpr int PPT = 2;             // output rows per thread (rows ty + h*PTY/PPT)
 constexpr int PNT = TX * PTY / PPT;  // phase threads per CTA
-// Resident CTAs per SM the phase kernel is built for: 2 in FP64 (its FP64
-// registers), 4 in FP32 (64 registers; 512^3: 1.57 -> 1.37 ms against 2).
-template <class T> __host__ __device__ constexpr int phase_min_blocks() { return sizeof(T) == 4 ? 4 : 2; }
+// Resident CTAs per SM the phase kernel is built for: 3 in FP64 (80 registers),
+// 4 in FP32 (64 registers; 512^3: 1.57 -> 1.37 ms against 2).
+template <class T> __host__ __device__ constexpr int phase_min_blocks() { return sizeof(T) == 4 ? 4 : 3; }
 
 // Momentum ring depth (planes per field): planes m-2 .. m+1, one in flight.
 // (A 5-plane ring with two planes in flight measured 30% slower on B200 at
@@ -209,20 +211,33 @@ template <class T, int TYv> struct MomGeo {
 static_assert(MomGeo<double, 8>::UX == 36 && MomGeo<double, 8>::EX == 36, "FP64 staged box widths");
 static_assert(MomGeo<float, 16>::UX == 40 && MomGeo<float, 16>::EX == 40, "FP32 staged box widths");
 
-// Staged phi planes of the phase kernel: the tile and its 2-cell ring in a
-// box starting XS cells (16 bytes) left of the tile, row pitch EX.
+// Staged planes of the phase kernel: phi on the tile and its 2-cell ring in a
+// box starting XS cells (16 bytes) left of the tile, row pitch EX, and u, v,
+// w on the cells the face fluxes need (u one more to the right, v one more
+// above).  Every staged array is a multiple of 128 bytes.
 template <class T> struct PhaseGeo {
   static constexpr int XS = 16 / (int)sizeof(T);
-  static constexpr int EX = (XS + TX + 2 + XS - 1) / XS * XS, EY = PTY + 4;
   static constexpr int AL = 128 / (int)sizeof(T);
+  static constexpr int EX = (XS + TX + 2 + XS - 1) / XS * XS, EY = PTY + 4;
   static constexpr int PSL = (EX * EY + AL - 1) / AL * AL;
-  static __host__ __device__ constexpr unsigned tx_bytes() { return (unsigned)(sizeof(T) * EX * EY); }
+  static constexpr int UW = (TX + 1 + XS - 1) / XS * XS;
+  static constexpr int UE = UW * PTY, VE = TX * (PTY + 1), WE = TX * PTY;
+  static constexpr int VOFF = (UE + AL - 1) / AL * AL, WOFF = VOFF + (VE + AL - 1) / AL * AL;
+  static constexpr int VSL = WOFF + (WE + AL - 1) / AL * AL;
+  static constexpr int FXE = PTY * (TX + 2), FYE = (PTY + 2) * TX;
+  static __host__ __device__ constexpr unsigned phi_bytes() { return (unsigned)(sizeof(T) * EX * EY); }
+  static __host__ __device__ constexpr unsigned vel_bytes() { return (unsigned)(sizeof(T) * (UE + VE + WE)); }
+  static __host__ __device__ constexpr size_t smem(int tab) {
+    return sizeof(T) * (size_t)(6 * PSL + FXE + FYE + 2 * VSL) + sizeof(double) * (tab + 3);
+  }
+  // the phi box of the tile inside the n x n plane
   static __host__ __device__ bool interior(int x0, int y0, int n) {
     return x0 >= XS && x0 - XS + EX <= n && y0 >= 2 && y0 + PTY + 2 <= n;
   }
 };
 static_assert(PhaseGeo<double>::EX == 36 && PhaseGeo<float>::EX == 40, "staged phi box widths");
-
+static_assert(PhaseGeo<double>::FXE % 16 == 0 && PhaseGeo<double>::FYE % 16 == 0, "128-byte aligned stages");
+static_assert(PhaseGeo<float>::FXE % 32 == 0 && PhaseGeo<float>::FYE % 32 == 0, "128-byte aligned stages");
 
 // 1/(sqrt(s) + tiny) for s > 0, the normalisation of A5.  With r = rsqrt(s),
 // 1/(sqrt(s) + tiny) = r/(1 + tiny*r) = r - tiny*r^2 + r*O((tiny*r)^2); the
@@ -236,33 +251,72 @@ __device__ __forceinline__ T inv_norm_plus(T s, T tiny) {
   return (T)1 / (sqrt(s) + tiny);
 }
 
-// phimap: a __grid_constant__ parameter (single simulation), or a map in the
-// ensemble's slot table (gmaps: acquired through the tensor-map proxy first).
-template <class T, bool TMA>
-__device__ __forceinline__ void phase_body(const StencilArgs<T>& a, int nz, int bx, int by, int bz,
-                                           const CUtensorMap* __restrict__ phimap, bool gmaps) {
+// One tile and z chunk of the phase-field update.
+//
+// Schedule at iteration m (stage m has landed: phi plane m, u and v of plane
+// m-1, w of plane m): psi(m) | barrier | F(m-1) | barrier | phi_new(m-2) and
+// the x, y part of plane m-1.  A thread owns its column (tx, ty + 8h): the z
+// neighbours of phi, F_z and w pass from plane to plane in registers, and
+// only F_x and F_y of the current plane go through shared memory.
+// The rings are 3 phi and 3 psi planes, one plane of F_x and F_y and two
+// velocity stages, 72 KB in FP64 with 78 registers: three CTAs per SM, where
+// the kernel was bound by latency at two (93 KB with 5 + 3 + 9 planes, 114
+// registers with the velocities prefetched into them).
+//
+// u, v and w arrive by tensor-map box loads on every tile; where the face
+// right of or above the tile wraps, its few values are read directly.  phi
+// arrives by a box load on the tiles whose box lies inside the grid
+// (tma_phi); on the others each thread copies the ring cells it computes psi
+// for with cp.async and periodic wrap.  Both fill the same shared cells.
+//
+// FP32 runs the loop over planes unrolled over the three ring slots, whose
+// addresses are then constants.  FP64 does not: its psi and F are four times
+// the instructions, and three copies of them stalled on instruction fetch
+// (5.2 of 12 cycles per issue).
+//
+// B200 against the kernel before (two CTAs per SM, velocities in registers, F
+// in nine shared planes): FP64 192^3 167 -> 147 us, 256^3 339 -> 307, 384^3 882
+// -> 755, 512^3 2260 -> 1920; FP32 512^3 1346 -> 1149; 96^3 and below unchanged.
+template <class T, bool SLOT>
+__device__ __forceinline__ void phase_body(const StencilArgs<T>& a, const T* __restrict__ phi_in,
+                                           T* __restrict__ phi_out, int nz, int bx, int by, int bz,
+                                           const PhaseMaps* __restrict__ maps) {
   if (a.ctrl->status) return;
   constexpr int TY = PTY, NT = PNT;
-  // The psi ring covers the tile and its 2-cell ring (LX x EY cells); phi and
-  // psi planes are stored with row pitch EX and the ring's first column at
-  // OFF (the staged phi box starts XS cells left of the tile, 16 bytes).
-  typedef PhaseGeo<T> PG;
-  constexpr int LX = TX + 4, EY = TY + 4, PE = LX * EY, EX = PG::EX, OFF = PG::XS - 2, SL = PG::PSL;
-  constexpr int FX = TX + 2, FY = TY + 2, FE = FX * FY;
+  typedef PhaseGeo<T> G;
+  constexpr int LX = TX + 4, PE = LX * G::EY, EX = G::EX, OFF = G::XS - 2, SL = G::PSL;
+  constexpr int FXP = TX + 2;  // row pitch of F_x (x = -1 .. TX)
   extern __shared__ __align__(128) unsigned char smem_raw[];
-  T* s_phi = reinterpret_cast<T*>(smem_raw);  // ring of 5 planes
-  T* s_psi = s_phi + 5 * SL;                  // ring of 3 planes
-  T* s_F = s_psi + 3 * SL;                    // ring of 3 planes x 3 components
-  double* s_tab = reinterpret_cast<double*>(s_F + 9 * FE);  // log table (FP64)
-  unsigned long long* s_bar = reinterpret_cast<unsigned long long*>(s_tab + PsiMath<T>::TAB);
-  for (int q = threadIdx.x; q < PsiMath<T>::TAB; q += NT) s_tab[q] = g_log_table[q];
-  if (PsiMath<T>::TAB) __syncthreads();
+  T* const s_phi = reinterpret_cast<T*>(smem_raw);
+  T* const s_psi = s_phi + 3 * SL;
+  T* const s_fx = s_psi + 3 * SL;
+  T* const s_fy = s_fx + G::FXE;
+  T* const s_vel = s_fy + G::FYE;  // two stages of u, v, w
+  double* const s_tab = reinterpret_cast<double*>(s_vel + 2 * G::VSL);
+  unsigned long long* const s_bar = reinterpret_cast<unsigned long long*>(s_tab + PsiMath<T>::TAB);
+  const int tid = threadIdx.x, tx = tid % TX, ty = tid / TX;
   const int n = a.c.n;
-  const T eps = (T)a.c.eps, epsi = (T)a.c.epsi, enumv = (T)a.c.enumv, tiny = (T)a.c.tiny;
-  const T dxi = (T)a.c.dxi, ddxi = (T)a.c.ddxi, dt = (T)a.c.dt, hdxi = (T)0.5 * dxi;
-  const T gamma = (T)(1.0 * a.ctrl->gumax);  // multi/main.f90:362
+  // z chunk bz of nz
+  const int x0 = bx * TX, y0 = by * TY, k0 = bz * n / nz, KZ = (bz + 1) * n / nz - k0;
+  const bool tma_phi = G::interior(x0, y0, n);
+  for (int q = tid; q < PsiMath<T>::TAB; q += NT) s_tab[q] = g_log_table[q];
+  if (tid == 0) {
+#pragma unroll
+    for (int q = 0; q < 3; ++q) mbar_init(s_bar + q, 1);
+    mbar_init_fence();
+    if (SLOT) {  // maps in the ensemble's slot table
+      tensormap_acquire(&maps->phi);
+      tensormap_acquire(&maps->u);
+      tensormap_acquire(&maps->v);
+      tensormap_acquire(&maps->w);
+    }
+  }
+  __syncthreads();
+  const T eps = (T)a.c.eps, enumv = (T)a.c.enumv, tiny = (T)a.c.tiny;
+  const T dt = (T)a.c.dt, hdxi = (T)(0.5 * a.c.dxi);
+  const double gamma = 1.0 * a.ctrl->gumax;  // multi/main.f90:362
+  const T gh = (T)(gamma * (0.5 * a.c.dxi)), ge = (T)(gamma * (a.c.eps * a.c.ddxi));
   const T mu = (T)a.ctrl->mean[0], mv = (T)a.ctrl->mean[1], mw = (T)a.ctrl->mean[2];
-  const int use_ident = a.c.tanh_identity;
   const T floor0 = a.c.phi_floor ? (T)0 : (T)-INFINITY;
   const T inv12e = (T)1 / ((T)1 + (T)2 * enumv);
   // psi where min(phi,1) is exactly 1 (drop interiors) or so small that both
@@ -273,202 +327,197 @@ __device__ __forceinline__ void phase_body(const StencilArgs<T>& a, int nz, int 
   // and the log is skipped -- bitwise the same values.
   const T psi0 = eps * PsiMath<T>::log_ratio((T)0 + enumv, (T)1 - (T)0 + enumv, s_tab);
   const T psi1 = eps * PsiMath<T>::log_ratio((T)1 + enumv, (T)1 - (T)1 + enumv, s_tab);
-  // z chunk bz of nz
-  const int x0 = bx * TX, y0 = by * TY, k0 = bz * n / nz, KZ = (bz + 1) * n / nz - k0;
-  const int tid = threadIdx.x, tx = tid % TX, ty = tid / TX;
-  constexpr int RY = TY / PPT;  // row step between a thread's output rows
-  const int i = x0 + tx;
-  const int ip = (i + 1 == n) ? 0 : i + 1;
   const size_t nn = (size_t)n * n;
-  // Each thread owns ring elements tid + r*NT of every plane (copy and psi)
-  // and F elements tid + r*NT; their in-plane offsets are the same on every
-  // plane, so they are computed once here.
-  constexpr int NPE = (PE + NT - 1) / NT, NFE = (FE + NT - 1) / NT;
-  int poff[NPE], fpe[NFE];
-#pragma unroll
-  for (int r = 0; r < NPE; ++r) {
-    const int e = min(tid + r * NT, PE - 1);
-    poff[r] = wrapi(x0 - 2 + e % LX, n) + n * wrapi(y0 - 2 + e / LX, n);
-  }
-#pragma unroll
-  for (int r = 0; r < NFE; ++r) {
-    const int e = min(tid + r * NT, FE - 1);
-    fpe[r] = (e % FX + 1 + OFF) + (e / FX + 1) * EX;
-  }
-  // stored index of the thread's ring element r
+  // Each thread owns ring elements tid + r*NT of every plane (copy and psi);
+  // pidx(r) is the stored index (row pitch EX, first column OFF).
+  constexpr int NPE = (PE + NT - 1) / NT;
   const auto pidx = [&](int r) {
     const int e = tid + r * NT;
     if constexpr (EX == LX && OFF == 0) return e;
     else return (e % LX + OFF) + (e / LX) * EX;
   };
-  // Tiles whose staged phi box lies inside the grid load each plane with one
-  // tensor-map box load; the edge tiles copy their elements with cp.async
-  // and wrap.  Both fill the same stored cells.
-  const bool tma = TMA && PG::interior(x0, y0, n);
-  int sp = 3;              // ring slot of plane m at iteration m
-  unsigned bar_phase = 0;  // bit s: parity of the next phase of slot s's barrier
-  if (tma) {
-    if (tid == 0) {
-#pragma unroll
-      for (int q = 0; q < 5; ++q) mbar_init(s_bar + q, 1);
-      mbar_init_fence();
-      if (gmaps) tensormap_acquire(phimap);
-    }
-    __syncthreads();
+  // Ring cells of F: F_x left and right of the tile, F_y below and above it,
+  // one each for threads 0 .. NRING-1.
+  constexpr int NRING = 2 * TY + 2 * TX;
+  const bool rx = tid < 2 * TY;
+  int rpe, rfe;  // plane index and F_x / F_y index of the thread's ring cell
+  {
+    const int q = rx ? tid : tid - 2 * TY;
+    const int ex = rx ? (q < TY ? -1 : TX) : q % TX, ey = rx ? q % TY : (q < TX ? -1 : TY);
+    rpe = (ex + 2 + OFF) + (ey + 2) * EX;
+    rfe = rx ? (ex + 1) + ey * FXP : ex + (ey + 1) * TX;
   }
-  // Ring slots by role, rotated once per plane (no per-plane index
-  // arithmetic): at iteration m the phi slots hold planes m-3 .. m+1 (m+1
-  // still in flight), the psi slots m-2 .. m (m being written), and the F
-  // slots m-3 .. m-1 (m-1 being written).
-  T *Phm3 = s_phi, *Phm2 = s_phi + SL, *Phm1 = s_phi + 2 * SL, *Ph0 = s_phi + 3 * SL, *Php1 = s_phi + 4 * SL;
-  T *PsW = s_psi, *Psm1 = s_psi + SL, *Psm2 = s_psi + 2 * SL;
-  T *FW = s_F, *Fm2 = s_F + 3 * FE, *Fm3 = s_F + 6 * FE;
-  int gij[PPT], gipj[PPT], gijp[PPT];
-#pragma unroll
-  for (int h = 0; h < PPT; ++h) {
-    const int j = y0 + ty + h * RY, jp = (j + 1 == n) ? 0 : j + 1;
-    gij[h] = i + n * j;
-    gipj[h] = ip + n * j;
-    gijp[h] = i + n * jp;
-  }
+  constexpr int RY = TY / PPT;
+  const int pe0 = (tx + 2 + OFF) + (ty + 2) * EX;  // own cell, row h: + h*RY*EX
+  const int fx0 = (tx + 1) + ty * FXP, fy0 = tx + (ty + 1) * TX;
+  const unsigned ij = (unsigned)(x0 + tx) + (unsigned)n * (unsigned)(y0 + ty);
+  const bool wrap_x = x0 + tx + 1 == n;
 
-  // phi plane m (2-cell ring) is copied into `dst` (ring slot `slot`) one
-  // iteration ahead of its use.
-  auto issue = [&](T* dst, int slot, int m) {
-    if (tma) {
-      if (tid == 0) {
-        mbar_arrive_expect_tx(s_bar + slot, PG::tx_bytes());
-        tma_load_2d(dst, phimap, x0 - PG::XS, wrapi(m, n) * n + y0 - 2, s_bar + slot);
+  // Stage j (m = k0 - 2 + j) into ring slot S: phi plane m; for 2 <= j <= KZ+2
+  // also u, v of plane m-1 and w of plane m into velocity stage j & 1.
+  auto issue = [&](int S, int j) {
+    const int m0 = wrapi(k0 - 2 + j, n), m1 = wrapi(k0 - 3 + j, n);
+    T* const dp = s_phi + S * SL;
+    const bool vel = j >= 2 && j <= KZ + 2;
+    if (tid == 0 && (tma_phi || vel)) {
+      unsigned long long* const bar = s_bar + S;
+      mbar_arrive_expect_tx(bar, (tma_phi ? G::phi_bytes() : 0u) + (vel ? G::vel_bytes() : 0u));
+      if (tma_phi) tma_load_2d(dp, &maps->phi, x0 - G::XS, m0 * n + y0 - 2, bar);
+      if (vel) {
+        T* const dv = s_vel + (j & 1) * G::VSL;
+        tma_load_2d(dv, &maps->u, x0, m1 * n + y0, bar);
+        tma_load_2d(dv + G::VOFF, &maps->v, x0, m1 * n + y0, bar);
+        tma_load_2d(dv + G::WOFF, &maps->w, x0, m0 * n + y0, bar);
       }
-      return;
     }
-    const T* src = a.phi_in + (size_t)wrapi(m, n) * nn;
+    if (!tma_phi) {
+      const T* const src = phi_in + nn * m0;
 #pragma unroll
-    for (int r = 0; r < NPE; ++r) {
-      const int e = tid + r * NT;
-      if (r < NPE - 1 || e < PE) cp_async_elem(dst + pidx(r), src + poff[r]);
+      for (int r = 0; r < NPE; ++r) {
+        const int e = tid + r * NT;
+        if (r < NPE - 1 || e < PE)
+          cp_async_elem(dp + pidx(r), src + (unsigned)(wrapi(x0 - 2 + e % LX, n) + n * wrapi(y0 - 2 + e / LX, n)));
+      }
+      cp_async_commit();
     }
-    cp_async_commit();
   };
-  issue(Ph0, sp, k0 - 2);
-  for (int m = k0 - 2; m <= k0 + KZ + 1; ++m) {
-    // plane m has landed: this thread's cp.async copies, or the slot's
-    // barrier phase for the box load (a wait that gives up records a timeout
-    // and carries on, so that no thread is left at a barrier)
-    if (tma) {
-      if (!mbar_wait(s_bar + sp, (bar_phase >> sp) & 1u, kWaitCycles)) atomicCAS(&a.ctrl->status, 0, kStatusTimeout);
-      bar_phase ^= 1u << sp;
-    } else {
-      cp_async_wait<0>();
-    }
-    const int spn = sp == 4 ? 0 : sp + 1;  // slot of plane m+1
-    // velocities of the output plane k = m-2, loaded now so that their latency
-    // hides behind the psi and F work below
-    T uc[PPT], uxp[PPT], vc[PPT], vyp[PPT], wc[PPT], wzp[PPT];
-    if (m >= k0 + 2) {
-      const size_t zo = nn * wrapi(m - 2, n), zop = nn * wrapi(m - 1, n);
+  // carried per own row: phi, F_z and w of the previous plane, and the part
+  // of the update that does not need F_z of the plane above
+  T c_[PPT], fz_[PPT], wc_[PPT], s_[PPT];
 #pragma unroll
-      for (int h = 0; h < PPT; ++h) {
-        uc[h] = a.u[zo + gij[h]];
-        uxp[h] = a.u[zo + gipj[h]];
-        vc[h] = a.v[zo + gij[h]];
-        vyp[h] = a.v[zo + gijp[h]];
-        wc[h] = a.w[zo + gij[h]];
-        wzp[h] = a.w[zop + gij[h]];
-      }
+  for (int h = 0; h < PPT; ++h) c_[h] = fz_[h] = wc_[h] = s_[h] = (T)0;
+  unsigned bar_phase = 0;  // bit s: parity of the next phase of slot s's barrier
+
+  auto iter = [&](const int S, const int j) __attribute__((always_inline)) {
+    const int Sm1 = S == 0 ? 2 : S - 1, Sm2 = S == 2 ? 0 : S + 1;  // slots of planes m-1, m-2
+    // plane m has landed: the slot's barrier phase for the box loads (a wait
+    // that gives up records a timeout and carries on, so that no thread is
+    // left at a barrier), or this thread's cp.async copies
+    if (tma_phi || (j >= 2 && j <= KZ + 2)) {
+      if (!mbar_wait(s_bar + S, (bar_phase >> S) & 1u, kWaitCycles)) atomicCAS(&a.ctrl->status, 0, kStatusTimeout);
+      bar_phase ^= 1u << S;
     }
-    // (1) psi of plane m on the elements this thread copied.
+    if (!tma_phi) cp_async_wait<0>();
+    const T *const Ph0 = s_phi + S * SL, *const Phm1 = s_phi + Sm1 * SL;
+    T* const Ps0 = s_psi + S * SL;
+    const T *const Psm1 = s_psi + Sm1 * SL, *const Psm2 = s_psi + Sm2 * SL;
+    // (1) psi of plane m on the elements this thread copied
 #pragma unroll
     for (int r = 0; r < NPE; ++r) {
-      const int e = tid + r * NT;
-      if (r < NPE - 1 || e < PE) {
+      if (r < NPE - 1 || tid + r * NT < PE) {
         const int ep = pidx(r);
         const T val = fmax(fmin(Ph0[ep], (T)1), floor0);
-        PsW[ep] = (val + enumv == enumv) ? psi0
+        Ps0[ep] = (val + enumv == enumv) ? psi0
                  : ((val == (T)1) ? psi1 : eps * PsiMath<T>::log_ratio(val + enumv, (T)1 - val + enumv, s_tab));
       }
     }
-    // psi of plane m is visible, and every thread is done with iteration m-1:
-    // the phi slot plane m+1 reuses (plane m-4, read by the last output) is
-    // free.  Two barriers per plane besides the F one, not three.
+    // psi(m) is visible and every thread is done with iteration m-1, so the
+    // phi slot of plane m-2 and the velocity stage that stage j+1 refills are free
     __syncthreads();
-    if (m + 1 <= k0 + KZ + 1) issue(Php1, spn, m + 1);
-    else cp_async_commit();
-    // (2) F on plane m-1 over the tile + 1 ring.
-    if (m >= k0) {
-      const T* Pc = Psm1;
-      const T* Pm = Psm2;
-      const T* Pp = PsW;
-      const T* Phc = Phm1;
-      T* F = FW;
+    if (j < KZ + 3) issue(Sm2, j + 1);
+    // (2) F on plane m-1: own cells (F_z stays in registers), then one ring cell
+    T fzc[PPT];
 #pragma unroll
-      for (int r = 0; r < NFE; ++r) {
-        const int e = tid + r * NT;
-        if (r == NFE - 1 && e >= FE) break;
-        const int pe = fpe[r];
-        const T gxv = Pc[pe + 1] - Pc[pe - 1];
-        const T gyv = Pc[pe + EX] - Pc[pe - EX];
-        const T gzv = Pp[pe] - Pm[pe];
-        if (gxv == (T)0 && gyv == (T)0 && gzv == (T)0) {  // uniform psi: n = 0 and F = 0 exactly
-          F[e] = (T)0;
-          F[FE + e] = (T)0;
-          F[2 * FE + e] = (T)0;
-          continue;
+    for (int h = 0; h < PPT; ++h) fzc[h] = (T)0;
+    if (j >= 2) {
+#pragma unroll
+      for (int r = 0; r <= PPT; ++r) {
+        if (r == PPT && tid >= NRING) break;
+        const int pe = r < PPT ? pe0 + r * RY * EX : rpe;
+        const T gxv = Psm1[pe + 1] - Psm1[pe - 1];
+        const T gyv = Psm1[pe + EX] - Psm1[pe - EX];
+        const T gzv = Ps0[pe] - Psm2[pe];
+        T fx = (T)0, fy = (T)0, fz = (T)0;
+        if (gxv != (T)0 || gyv != (T)0 || gzv != (T)0) {  // uniform psi: n = 0 and F = 0 exactly
+          const T normod = inv_norm_plus(fma(gzv, gzv, fma(gyv, gyv, gxv * gxv)), tiny);
+          T t;
+          if (a.c.tanh_identity) {
+            // tanh(0.5*log(a/b)) = (a-b)/(a+b) with a = val+enum, b = 1-val+enum
+            const T val = fmax(fmin(Phm1[pe], (T)1), floor0);
+            t = ((T)2 * val - (T)1) * inv12e;
+          } else {
+            t = tanh((T)0.5 * Psm1[pe] * (T)a.c.epsi);
+          }
+          const T g = (T)0.25 * ((T)1 - t * t);
+          fx = g * (gxv * normod);
+          fy = g * (gyv * normod);
+          fz = g * (gzv * normod);
         }
-        const T normod = inv_norm_plus(gxv * gxv + gyv * gyv + gzv * gzv, tiny);
-        T t;
-        if (use_ident) {
-          // tanh(0.5*log(a/b)) = (a-b)/(a+b) with a = val+enum, b = 1-val+enum
-          const T val = fmax(fmin(Phc[pe], (T)1), floor0);
-          t = ((T)2 * val - (T)1) * inv12e;
+        if (r < PPT) {
+          s_fx[fx0 + r * RY * FXP] = fx;
+          s_fy[fy0 + r * RY * TX] = fy;
+          fzc[r < PPT ? r : 0] = fz;
+        } else if (rx) {
+          s_fx[rfe] = fx;
         } else {
-          t = tanh((T)0.5 * Pc[pe] * epsi);
+          s_fy[rfe] = fy;
         }
-        const T g = (T)0.25 * ((T)1 - t * t);
-        F[e] = g * (gxv * normod);
-        F[FE + e] = g * (gyv * normod);
-        F[2 * FE + e] = g * (gzv * normod);
       }
     }
     __syncthreads();
-    // (3) output plane k = m-2.
-    if (m >= k0 + 2) {
-      const T* P0 = Phm2;
-      const T* Pm1 = Phm3;
-      const T* Pp1 = Phm1;
-      const T* F0 = Fm2;
-      const T* Fm = Fm3;
-      const T* Fp = FW;
+    if (j >= 2) {
+      // (3) phi_new of plane m-2, then the x, y part of plane m-1
+      const T* const V = s_vel + (j & 1) * G::VSL;
+      const int k = k0 - 3 + j;  // plane m-1
+      if (j >= 4) {
+        T* const out = phi_out + nn * (k - 1);
+#pragma unroll
+        for (int h = 0; h < PPT; ++h) out[ij + (unsigned)(h * RY * n)] = fma(dt, fma(-gh, fzc[h], s_[h]), c_[h]);
+      }
 #pragma unroll
       for (int h = 0; h < PPT; ++h) {
-        const int pe = (tx + 2 + OFF) + (ty + h * RY + 2) * EX;
-        const int fe = (tx + 1) + (ty + h * RY + 1) * FX;
-        const T c = P0[pe], pxp = P0[pe + 1], pxm = P0[pe - 1], pyp = P0[pe + EX], pym = P0[pe - EX];
-        const T pzp = Pp1[pe], pzm = Pm1[pe];
-        const size_t g = nn * wrapi(m - 2, n) + gij[h];
-        const T uc_ = uc[h] - mu, uxp_ = uxp[h] - mu, vc_ = vc[h] - mv, vyp_ = vyp[h] - mv;
-        const T wc_ = wc[h] - mw, wzp_ = wzp[h] - mw;
-        // The factors 0.5 of the face averages and central differences are
-        // folded into hdxi = 0.5*dxi: scaling by a power of 2 commutes with
-        // rounding, so every term is bitwise the reference's (x*0.5*y - ..)*dxi.
-        T r = -(uxp_ * (pxp + c) - uc_ * (c + pxm)) * hdxi - (vyp_ * (pyp + c) - vc_ * (c + pym)) * hdxi -
-              (wzp_ * (pzp + c) - wc_ * (c + pzm)) * hdxi;
-        r = r + gamma * (eps * (pxp - (T)2 * c + pxm) * ddxi + eps * (pyp - (T)2 * c + pym) * ddxi +
-                         eps * (pzp - (T)2 * c + pzm) * ddxi);
-        r = r - gamma * ((F0[fe + 1] - F0[fe - 1]) * hdxi + (F0[FE + fe + FX] - F0[FE + fe - FX]) * hdxi +
-                         (Fp[2 * FE + fe] - Fm[2 * FE + fe]) * hdxi);
-        a.phi_out[g] = c + dt * r;
+        const int pe = pe0 + h * RY * EX, row = ty + h * RY;
+        const T c = Phm1[pe];
+        if (j <= KZ + 2) {
+          const T wzp = V[G::WOFF + tx + row * TX] - mw;
+          if (j >= 3) {
+            T uxp = V[tx + 1 + row * G::UW], vyp = V[G::VOFF + tx + (row + 1) * TX];
+            if (wrap_x) uxp = a.u[nn * k + (unsigned)n * (unsigned)(y0 + row)];
+            if (y0 + row + 1 == n) vyp = a.v[nn * k + (unsigned)(x0 + tx)];
+            uxp -= mu;
+            vyp -= mv;
+            const T uc = V[tx + row * G::UW] - mu, vc = V[G::VOFF + tx + row * TX] - mv;
+            const T pxp = Phm1[pe + 1], pxm = Phm1[pe - 1], pyp = Phm1[pe + EX], pym = Phm1[pe - EX];
+            const T pzp = Ph0[pe], pzm = c_[h];
+            const int fx = fx0 + h * RY * FXP, fy = fy0 + h * RY * TX;
+            // The factors 0.5 of the face averages and central differences
+            // are folded into hdxi = 0.5*dxi and gh = gamma*hdxi.  The fused
+            // multiply-adds are written out, so that every instantiation (a
+            // slot of the ensemble among them) rounds alike.
+            T conv = uxp * (pxp + c);
+            conv = fma(-uc, c + pxm, conv);
+            conv = fma(vyp, pyp + c, conv);
+            conv = fma(-vc, c + pym, conv);
+            conv = fma(wzp, pzp + c, conv);
+            conv = fma(-wc_[h], c + pzm, conv);
+            const T lap = (pxp - (T)2 * c + pxm) + (pyp - (T)2 * c + pym) + (pzp - (T)2 * c + pzm);
+            const T div = (s_fx[fx + 1] - s_fx[fx - 1]) + (s_fy[fy + TX] - s_fy[fy - TX]) - fz_[h];
+            s_[h] = fma(-gh, div, fma(-hdxi, conv, ge * lap));
+          }
+          wc_[h] = wzp;
+        }
+        c_[h] = c;
+        fz_[h] = fzc[h];
       }
     }
-    // rotate the rings for plane m+1: the slot of the oldest plane of each
-    // ring takes the next plane
-    T* t = Phm3;
-    Phm3 = Phm2; Phm2 = Phm1; Phm1 = Ph0; Ph0 = Php1; Php1 = t;
-    sp = spn;
-    t = Psm2;
-    Psm2 = Psm1; Psm1 = PsW; PsW = t;
-    t = Fm3;
-    Fm3 = Fm2; Fm2 = FW; FW = t;
+  };
+  issue(0, 0);
+  if constexpr (sizeof(T) == 4) {
+#pragma unroll 1
+    for (int j = 0; j <= KZ + 3; j += 3) {
+      iter(0, j);
+      if (j + 1 > KZ + 3) break;
+      iter(1, j + 1);
+      if (j + 2 > KZ + 3) break;
+      iter(2, j + 2);
+    }
+  } else {
+    int S = 0;
+#pragma unroll 1
+    for (int j = 0; j <= KZ + 3; ++j) {
+      iter(S, j);
+      S = S == 2 ? 0 : S + 1;
+    }
   }
 }
 
@@ -982,8 +1031,8 @@ constexpr int FNT = 1024;  // threads of the FP32 refinement form's finalize
 // Single simulation: block coordinates are the grid's.
 template <class T>
 __global__ void __launch_bounds__(PNT, phase_min_blocks<T>())
-    phase_kernel(StencilArgs<T> a, const __grid_constant__ CUtensorMap phimap) {
-  phase_body<T, true>(a, gridDim.z, blockIdx.x, blockIdx.y, blockIdx.z, &phimap, false);
+    phase_kernel(const __grid_constant__ StencilArgs<T> a, const __grid_constant__ PhaseMaps maps) {
+  phase_body<T, false>(a, a.phi_in, a.phi_out, gridDim.z, blockIdx.x, blockIdx.y, blockIdx.z, &maps);
 }
 template <class T, bool PF, int MTYv>
 __global__ void __launch_bounds__(TX * 8, momentum_min_blocks<T>(PF, MTYv))
@@ -1014,11 +1063,18 @@ template <class T>
 __global__ void __launch_bounds__(PNT, phase_min_blocks<T>()) phase_kernel_b(const SlotArgs<T>* __restrict__ slots, int zch) {
   const int sl = blockIdx.z / zch;
   if (!slots[sl].active) return;
-  StencilArgs<T> a = slots[sl].st;
+  // The slot's arguments are copied to shared memory once per CTA: the single
+  // simulation reads them from its kernel parameters, and holding them in
+  // registers spills.
+  __shared__ alignas(StencilArgs<T>) unsigned sa[sizeof(StencilArgs<T>) / 4];
+  static_assert(sizeof(StencilArgs<T>) % 4 == 0, "copied by words");
+  const unsigned* const src = reinterpret_cast<const unsigned*>(&slots[sl].st);
+  for (unsigned q = threadIdx.x; q < sizeof(sa) / 4; q += PNT) sa[q] = src[q];
+  __syncthreads();
+  const StencilArgs<T>& a = *reinterpret_cast<const StencilArgs<T>*>(sa);
   const int par = (int)(a.ctrl->nstep & 1);
-  a.phi_in = slots[sl].phi[par];
-  a.phi_out = slots[sl].phi[par ^ 1];
-  phase_body<T, true>(a, zch, blockIdx.x, blockIdx.y, blockIdx.z - sl * zch, &slots[sl].maps.phase_phi[par], true);
+  phase_body<T, true>(a, slots[sl].phi[par], slots[sl].phi[par ^ 1], zch, blockIdx.x, blockIdx.y,
+                      blockIdx.z - sl * zch, &slots[sl].maps.phase[par]);
 }
 template <class T, bool PF, int MTYv>
 __global__ void __launch_bounds__(TX * 8, momentum_min_blocks<T>(PF, MTYv)) momentum_kernel_b(const SlotArgs<T>* __restrict__ slots, int zch) {
@@ -1084,10 +1140,7 @@ __global__ void materialize_kernel(T* u, T* v, T* w, size_t count, Ctrl* ctrl) {
 }
 
 // ============================================================ launchers
-template <class T> static size_t phase_smem() {
-  return sizeof(T) * (size_t)(8 * PhaseGeo<T>::PSL + 9 * (TX + 2) * (PTY + 2)) +
-         sizeof(double) * (PsiMath<T>::TAB + 5);
-}
+template <class T> static size_t phase_smem() { return PhaseGeo<T>::smem(PsiMath<T>::TAB); }
 template <class T> static size_t momentum_smem(bool pf, int mty) {
   const int ns = momentum_ring(mty);
   const size_t b = mty == 8 ? MomGeo<T, 8>::bar_offset(pf, ns) : MomGeo<T, 16>::bar_offset(pf, ns);
@@ -1155,8 +1208,18 @@ template <class T, int TYv> static cudaError_t momentum_maps(PlaneMaps* pm, cons
   return cudaSuccess;
 }
 
+template <class T> static cudaError_t phase_maps(PhaseMaps* pm, const StencilArgs<T>& a) {
+  typedef PhaseGeo<T> G;
+  const int n = a.c.n;
+  cudaError_t e;
+  if ((e = plane_map(&pm->phi, a.phi_in, n, G::EX, G::EY))) return e;
+  if ((e = plane_map(&pm->u, a.u, n, G::UW, PTY))) return e;
+  if ((e = plane_map(&pm->v, a.v, n, TX, PTY + 1))) return e;
+  return plane_map(&pm->w, a.w, n, TX, PTY);
+}
+
 // A served-ensemble slot's tensor maps: the momentum boxes for both tile
-// heights and both phi parities, the phase kernel's phi box per parity, and
+// heights and both phi parities, the phase kernel's boxes per parity, and
 // the column passes' spectrum views.
 template <class T> cudaError_t encode_slot_maps(SlotArgs<T>* s, int n, bool pf) {
   cudaError_t e;
@@ -1166,7 +1229,7 @@ template <class T> cudaError_t encode_slot_maps(SlotArgs<T>* s, int n, bool pf) 
     a.phi_in = pf ? s->phi[par] : nullptr;
     if ((e = momentum_maps<T, 8>(&s->maps.mom[0][par], a, pf))) return e;
     if ((e = momentum_maps<T, 16>(&s->maps.mom[1][par], a, pf))) return e;
-    if (pf && (e = plane_map(&s->maps.phase_phi[par], s->phi[par], n, PhaseGeo<T>::EX, PTY + 4))) return e;
+    if (pf && (e = phase_maps(&s->maps.phase[par], a))) return e;
   }
   return encode_column_maps<T>(&s->maps, s->po.spec, n);
 }
@@ -1210,8 +1273,8 @@ template <class T> cudaError_t launch_phase(const StencilArgs<T>& a, cudaStream_
   const int n = a.c.n;
   const int tiles = (n / TX) * (n / PTY);
   dim3 grid(n / TX, n / PTY, kz > 0 ? n / kz : pick_chunks(n, tiles, phase_min_blocks<T>() * sm_count(), 4));
-  CUtensorMap pm;
-  cudaError_t e = plane_map(&pm, a.phi_in, n, PhaseGeo<T>::EX, PTY + 4);
+  PhaseMaps pm;
+  cudaError_t e = phase_maps(&pm, a);
   if (e) return e;
   phase_kernel<T><<<grid, PNT, phase_smem<T>(), st>>>(a, pm);
   return cudaGetLastError();
