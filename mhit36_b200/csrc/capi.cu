@@ -183,7 +183,7 @@ typedef std::pair<const char*, std::function<cudaError_t()>> Stage;
 //   FP64: [phase] momentum xfwd yfwd zsolve yinv xinv project
 //   FP32 refine: [phase] momentum, solve 1 (xfwd yfwd zsolve yinv xinv -> p0),
 //     solve 2 of the FP64 residual (xres yfwd2 zsolve2 yinv2 xinv2 -> dp),
-//     project (FP64) [finalize]
+//     project (FP64) [finalize, where the projection does not end the step]
 std::vector<Stage> step_stages(mhit_handle* h, int cur) {
   std::vector<Stage> v;
   cudaStream_t st = h->st;
@@ -232,10 +232,12 @@ std::vector<Stage> step_stages(mhit_handle* h, int cur) {
     for (int k = 0; k < (fused ? 4 : 5); ++k)
       v.push_back({rnames[k], [pr, n, k, st] { return mhit::launch_poisson_stage<float>(n, pr, k, st); }});
     float* dp = h->fdp;
-    if (fused)
+    if (fused) {
       v.push_back({"xinvproj", [pr, a, n, st] { return mhit::launch_xinv_project<float>(n, pr, a, st); }});
-    else
+    } else {
       v.push_back({"project", [a, dp, st] { return mhit::launch_project_refine(a, dp, st); }});
+      v.push_back({"finalize", [a, st] { return mhit::launch_finalize_refine(a, st); }});
+    }
   }
   return v;
 }
