@@ -39,6 +39,17 @@ __device__ __forceinline__ size_t gidx(int i, int j, int k, int n) {
   return (size_t)i + (size_t)n * ((size_t)j + (size_t)n * (size_t)k);
 }
 
+// ---- dependent launches ----
+// First in every kernel that launch_dep may launch: lets the next kernel's
+// CTAs be scheduled once every CTA of this one is here, and returns when the
+// kernel before has finished and its results are visible.  Every thread calls
+// it, so a kernel that has finished implies that all before it have.  Without
+// the launch attribute it returns at once.
+__device__ __forceinline__ void dep_begin() {
+  asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
+  asm volatile("griddepcontrol.wait;\n" ::: "memory");
+}
+
 // ---- asynchronous global -> shared copies (sm_80+ cp.async) ----
 // One element per call (4 or 8 bytes); a thread's copies land in issue
 // order groups: commit after a batch, wait until at most N groups are pending.

@@ -24,6 +24,7 @@ template <class T> struct PoissonArgs {
   double cdiv = 0;         // rho*dxi/dt
   const T* pres = nullptr;  // refinement: first-solve pressure p0 (residual RHS) or nullptr
   double ddxi = 0;         // 1/dx^2 for the residual Laplacian
+  const CUtensorMap* col_maps = nullptr;  // the column passes' views of spec (y, z), if already encoded
 };
 
 template <class T> cudaError_t launch_poisson(int n, const PoissonArgs<T>& a, cudaStream_t st);
@@ -136,8 +137,8 @@ cudaError_t encode_tensor_map(CUtensorMap* m, int rank, const void* base, const 
                               const uint64_t* strides, const uint32_t* box, int elem_bytes = 8);
 // A slot's tensor maps from its table entry's field pointers (n^3 grid).
 template <class T> cudaError_t encode_slot_maps(SlotArgs<T>* a, int n, bool phase_field);
-// The column passes' spectrum views of a slot (part of encode_slot_maps).
-template <class T> cudaError_t encode_column_maps(SlotMaps* m, const void* spec, int n);
+// The column passes' spectrum views (y passes, z solve).
+template <class T> cudaError_t encode_column_maps(CUtensorMap* y, CUtensorMap* z, const void* spec, int n);
 // One-warp self-check of the bounded barrier wait (writes 0 or MHIT_ERR_TIMEOUT).
 cudaError_t launch_wait_check(int arrive, long long limit_cycles, int* out_dev, cudaStream_t st);
 cudaError_t launch_refine_divergence(const StencilArgs<float>& a, const float* dp, double* out, cudaStream_t st);

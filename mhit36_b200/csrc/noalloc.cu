@@ -77,6 +77,7 @@ struct Addrs {
   double2* spec = nullptr;
   double2* tw = nullptr;
   double* k2 = nullptr;
+  CUtensorMap maps[kSizeSlots][2];  // the column passes' views of spec at each size
 };
 Addrs g_addrs[kMaxDevices];
 std::mutex g_mutex;
@@ -124,7 +125,7 @@ void host_tables(std::vector<double2>& tw, std::vector<double>& k2) {
   }
 }
 
-int setup_device(int dev, Addrs* out) {
+int setup_device(int dev, const Addrs** out) {
   std::lock_guard<std::mutex> lock(g_mutex);
   Addrs& a = g_addrs[dev];
   if (!a.ready) {
@@ -140,11 +141,13 @@ int setup_device(int dev, Addrs* out) {
     if (cudaMemcpy(t.k2, k2.data(), k2.size() * sizeof(double), cudaMemcpyHostToDevice) != cudaSuccess)
       return MHIT_ERR_CUDA;
     for (int q = 0; q < kSizes.count; ++q)
-      if (mhit::prepare_poisson(kSizes.n[q]) != cudaSuccess) return MHIT_ERR_CUDA;
+      if (mhit::prepare_poisson(kSizes.n[q]) != cudaSuccess ||
+          mhit::encode_column_maps<double>(&t.maps[q][0], &t.maps[q][1], t.spec, kSizes.n[q]) != cudaSuccess)
+        return MHIT_ERR_CUDA;
     t.ready = true;
     a = t;
   }
-  *out = a;
+  *out = &a;  // not written again once ready
   return MHIT_OK;
 }
 
@@ -159,9 +162,10 @@ extern "C" int mhit_poisson_noalloc(const double* rhs_dev, double* p_dev, int n,
   if (mhit::spectrum_pitch(n, 0) > kPitchMax) return MHIT_ERR_SCRATCH_LIMIT;
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices) return MHIT_ERR_CUDA;
-  Addrs a;
-  int rc = setup_device(dev, &a);
+  const Addrs* ap = nullptr;
+  int rc = setup_device(dev, &ap);
   if (rc) return rc;
+  const Addrs& a = *ap;
   mhit::PoissonArgs<double> pa;
   pa.rhs = rhs_dev;
   pa.spec = a.spec;
@@ -169,6 +173,7 @@ extern "C" int mhit_poisson_noalloc(const double* rhs_dev, double* p_dev, int n,
   pa.tw = a.tw + kSizes.off[slot];
   pa.k2tab = a.k2 + (size_t)mode_index(k2_mode, grid_mode) * kSizes.total + kSizes.off[slot];
   pa.ctrl = nullptr;
+  pa.col_maps = a.maps[slot];
   if (mhit::launch_poisson<double>(n, pa, static_cast<cudaStream_t>(stream)) != cudaSuccess) return MHIT_ERR_CUDA;
   return MHIT_OK;
 }

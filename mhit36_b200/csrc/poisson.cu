@@ -321,13 +321,14 @@ __device__ __forceinline__ void rcol_run(int total, const typename C2<T>::t* __r
   }
 }
 
-template <int N, int KIND, class T>
+template <int N, int KIND, class T, bool DEP = false>
 __global__ void __launch_bounds__(RCfg<N, T>::NT, RCfg<N, T>::minb(KIND)) rcol_kernel(typename C2<T>::t* __restrict__ spec,
                                                               const typename C2<T>::t* __restrict__ tw,
                                                               const double* __restrict__ k2tab,
                                                               const Ctrl* __restrict__ ctrl,
                                                               const __grid_constant__ CUtensorMap map) {
   typedef PCfg<N, T> G;
+  if (DEP) dep_begin();
   constexpr bool PFS = RCfg<N, T>::pf_single(KIND);
   rcol_run<N, KIND, T, PFS, PFS>(G::NCHUNK * N, tw, [&](int it) {
     ColSlab s = slab_single<N, KIND, T>(spec, tw, k2tab, ctrl, it);
@@ -378,6 +379,14 @@ template <int N, class T> struct XCfg {
   static constexpr int LS = sizeof(T) == 8 ? reg_rows(N) : N;
   static __device__ __forceinline__ int slot(int n) { return sizeof(T) == 8 ? reg_pad(n) : reg_swz(n); }
 };
+
+// Stand-alone solves whose kernels are launched so that each may start while
+// the one before it drains: up to 128^3, where a solve is bound by launch
+// latency (B200: 64^3 22.5 -> 18 us, 128^3 52.9 -> 49.5).  At 384^3 the waiting
+// CTAs cost more than that gains (1256 -> 1438), and in the step's CUDA graph
+// the same launches are slower at every size (64^3 59.5 -> 61.7, 512^3 9.6 ->
+// 10.0 ms), so those kernels are instances of their own.
+__host__ __device__ constexpr bool dep_solve(int n) { return n <= 128; }
 
 template <int N, class T>
 __device__ __forceinline__ void xinv_reg_body(const typename C2<T>::t* __restrict__ spec, T* __restrict__ p,
@@ -734,12 +743,14 @@ __global__ void __launch_bounds__(256, xfwd_min_blocks<N, MODE, T>()) xfwd_kerne
                                                   const T* __restrict__ p0, typename C2<T>::t* __restrict__ spec,
                                                   const typename C2<T>::t* __restrict__ tw,
                                                   const Ctrl* __restrict__ ctrl, double cdiv, double ddxi) {
+  if (MODE == 1 && dep_solve(N)) dep_begin();
   xfwd_reg_body<N, MODE, T>(us, vs, ws, rhs, p0, spec, tw, ctrl, cdiv, ddxi, blockIdx.x, blockIdx.y);
 }
-template <int N, class T>
+template <int N, class T, bool DEP = false>
 __global__ void __launch_bounds__(256, reg_elems(N) == 8 ? 3 : 2) xinv_kernel(const typename C2<T>::t* __restrict__ spec, T* __restrict__ p,
                                                   const typename C2<T>::t* __restrict__ tw,
                                                   const Ctrl* __restrict__ ctrl) {
+  if (DEP) dep_begin();
   xinv_reg_body<N, T>(spec, p, tw, ctrl, blockIdx.x, blockIdx.y);
 }
 
@@ -810,14 +821,39 @@ template <int N, int KIND, class T> static cudaError_t col_map(CUtensorMap* map,
   return encode_tensor_map(map, 2, spec, dims, strides, box, (int)sizeof(T));
 }
 
-template <int N, int KIND, class T> static void launch_col(const PoissonArgs<T>& a, cudaStream_t st) {
+// Launch a kernel that starts with dep_begin, which may start before the kernel
+// ahead of it on the stream has finished.
+template <class... K, class... A>
+static void launch_dep(void (*kernel)(K...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A&&... args) {
+  cudaLaunchAttribute at;
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cfg.attrs = &at;
+  cfg.numAttrs = 1;
+  cudaLaunchKernelEx(&cfg, kernel, K(args)...);
+}
+
+// DEP: as part of a stand-alone solve of dependent launches.
+template <int N, int KIND, class T, bool DEP = false>
+static void launch_col(const PoissonArgs<T>& a, cudaStream_t st) {
   CUtensorMap map;
-  if (col_map<N, KIND, T>(&map, a.spec)) {  // surfaces as the launch error of an empty grid
+  if (a.col_maps) {
+    map = a.col_maps[KIND == 2 ? 1 : 0];
+  } else if (col_map<N, KIND, T>(&map, a.spec)) {  // surfaces as the launch error of an empty grid
     rcol_kernel<N, KIND, T><<<0, 1, 0, st>>>(a.spec, a.tw, a.k2tab, a.ctrl, map);
     return;
   }
-  rcol_kernel<N, KIND, T><<<rcolgrid<N, KIND, T, false>(), RCfg<N, T>::NT, rcolsmem<N, KIND, T>(), st>>>(
-      a.spec, a.tw, a.k2tab, a.ctrl, map);
+  const int grid = rcolgrid<N, KIND, T, false>();
+  const size_t sm = rcolsmem<N, KIND, T>();
+  if constexpr (DEP)
+    launch_dep(rcol_kernel<N, KIND, T, true>, grid, RCfg<N, T>::NT, sm, st, a.spec, a.tw, a.k2tab, a.ctrl, map);
+  else
+    rcol_kernel<N, KIND, T><<<grid, RCfg<N, T>::NT, sm, st>>>(a.spec, a.tw, a.k2tab, a.ctrl, map);
 }
 template <int N, int KIND, class T>
 static void launch_col_b(const SlotArgs<T>* slots, int nslots, int which, cudaStream_t st) {
@@ -847,6 +883,12 @@ template <int N, class T> static cudaError_t set_attrs() {
     if ((e = cudaFuncSetAttribute(rcol_kernel<N, 0, T>, A, q0))) return e;
     if ((e = cudaFuncSetAttribute(rcol_kernel<N, 1, T>, A, q1))) return e;
     if ((e = cudaFuncSetAttribute(rcol_kernel<N, 2, T>, A, q2))) return e;
+    if constexpr (dep_solve(N)) {
+      if ((e = cudaFuncSetAttribute(rcol_kernel<N, 0, T, true>, A, q0))) return e;
+      if ((e = cudaFuncSetAttribute(rcol_kernel<N, 1, T, true>, A, q1))) return e;
+      if ((e = cudaFuncSetAttribute(rcol_kernel<N, 2, T, true>, A, q2))) return e;
+      if ((e = cudaFuncSetAttribute(xinv_kernel<N, T, true>, A, xs))) return e;
+    }
     if ((e = cudaFuncSetAttribute(rcol_kernel_b<N, 0, T>, A, r0))) return e;
     if ((e = cudaFuncSetAttribute(rcol_kernel_b<N, 1, T>, A, r1))) return e;
     if ((e = cudaFuncSetAttribute(rcol_kernel_b<N, 2, T>, A, r2))) return e;
@@ -881,11 +923,15 @@ static cudaError_t poisson_run(const PoissonArgs<T>& a, cudaStream_t st) {
   typedef PCfg<N, T> G;
   const dim3 gx(N / (2 * G::P), N);
   const size_t xs = xsmem<N, T>();
+  constexpr bool DEP = dep_solve(N);
   launch_xfwd<N, T>(a, st);
-  launch_col<N, 0, T>(a, st);
-  launch_col<N, 2, T>(a, st);
-  launch_col<N, 1, T>(a, st);
-  xinv_kernel<N, T><<<gx, XCfg<N, T>::NT, xs, st>>>(a.spec, a.p, a.tw, a.ctrl);
+  launch_col<N, 0, T, DEP>(a, st);
+  launch_col<N, 2, T, DEP>(a, st);
+  launch_col<N, 1, T, DEP>(a, st);
+  if constexpr (DEP)
+    launch_dep(xinv_kernel<N, T, true>, gx, XCfg<N, T>::NT, xs, st, a.spec, a.p, a.tw, a.ctrl);
+  else
+    xinv_kernel<N, T><<<gx, XCfg<N, T>::NT, xs, st>>>(a.spec, a.p, a.tw, a.ctrl);
   return cudaGetLastError();
 }
 
@@ -936,21 +982,21 @@ cudaError_t launch_poisson_stage(int n, const PoissonArgs<T>& a, int stage, cuda
       return cudaErrorInvalidValue;
   }
 }
-template <class T> cudaError_t encode_column_maps(SlotMaps* m, const void* spec, int n) {
+template <class T> cudaError_t encode_column_maps(CUtensorMap* y, CUtensorMap* z, const void* spec, int n) {
   cudaError_t e;
   switch (n) {
 #define CM_CASE(NN)                                                        \
   case NN:                                                                 \
-    if ((e = col_map<NN, 0, T>(&m->col_y, spec))) return e;                \
-    return col_map<NN, 2, T>(&m->col_z, spec);
+    if ((e = col_map<NN, 0, T>(y, spec))) return e;                        \
+    return col_map<NN, 2, T>(z, spec);
     MHIT_FOR_SIZES(CM_CASE)
 #undef CM_CASE
     default:
       return cudaErrorInvalidValue;
   }
 }
-template cudaError_t encode_column_maps<double>(SlotMaps*, const void*, int);
-template cudaError_t encode_column_maps<float>(SlotMaps*, const void*, int);
+template cudaError_t encode_column_maps<double>(CUtensorMap*, CUtensorMap*, const void*, int);
+template cudaError_t encode_column_maps<float>(CUtensorMap*, CUtensorMap*, const void*, int);
 
 template cudaError_t launch_poisson_stage<double>(int, const PoissonArgs<double>&, int, cudaStream_t);
 template cudaError_t launch_poisson_stage<float>(int, const PoissonArgs<float>&, int, cudaStream_t);

@@ -1231,7 +1231,7 @@ template <class T> cudaError_t encode_slot_maps(SlotArgs<T>* s, int n, bool pf) 
     if ((e = momentum_maps<T, 16>(&s->maps.mom[1][par], a, pf))) return e;
     if (pf && (e = phase_maps(&s->maps.phase[par], a))) return e;
   }
-  return encode_column_maps<T>(&s->maps, s->po.spec, n);
+  return encode_column_maps<T>(&s->maps.col_y, &s->maps.col_z, s->po.spec, n);
 }
 template cudaError_t encode_slot_maps<double>(SlotArgs<double>*, int, bool);
 template cudaError_t encode_slot_maps<float>(SlotArgs<float>*, int, bool);
