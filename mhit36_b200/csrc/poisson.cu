@@ -34,7 +34,14 @@ template <int N, class T = double> struct PCfg {
   // chunk is still a 64-128-byte row segment of the half spectrum (measured
   // 20-25% faster on B200 at 512^3; the x passes are faster with 2048/N).
   static constexpr int L = (N <= 256) ? 8 : ((N <= 512) ? 4 : 2);
-  static constexpr int P = L;                               // line pairs per CTA (x passes)
+  // Line pairs per CTA of the x passes.  Half a column chunk from 192 up: the
+  // same threads per SM in twice the CTAs wait at barriers of half the warps
+  // (B200, forward/residual/inverse: FP32 512^3 441/728/247 -> 414/703/237 us,
+  // 384^3 222/313/117 -> 205/296/117; FP64 256^3 forward 130 -> 126, 384^3
+  // 377/-/225 -> 368/-/220, 512^3 unchanged).  A quarter: 384^3 FP32 205 -> 208,
+  // 117 -> 121.  Up to 128^3 CTAs are too few to split, and at 768 and 1024 half
+  // a chunk is one pair, which reads every other line of v twice.
+  static constexpr int P = (N >= 192 && N <= 512) ? L / 2 : L;
   static constexpr int CC = (sizeof(T) == 8) ? L : 2 * L;   // kx columns per CTA (y/z passes)
   static constexpr int PITCH = ((N / 2 + 1) + CC - 1) / CC * CC;
   static constexpr int NCHUNK = PITCH / CC;
@@ -514,7 +521,7 @@ __device__ __forceinline__ void xfwd_reg_body(const T* __restrict__ us, const T*
 //     inverse and projection.
 template <int N, class T> struct XPCfg {
   static constexpr bool ON = (N & (N - 1)) == 0 && N >= 256;  // power-of-two sizes (8 elements per thread)
-  static constexpr int P = PCfg<N, T>::P;
+  static constexpr int P = PCfg<N, T>::L;
   static constexpr int TPC = N / 8;
   static constexpr int NT = (P + 1) * TPC;  // a multiple of 32 for N >= 256
   static constexpr int KZ = N >= 512 ? 16 : 8;
@@ -731,14 +738,20 @@ __global__ void __launch_bounds__(XPCfg<N, T>::NT, 2) xinvproj_kernel_b(const Sl
 
 // ---------------------------------------------------------------- entry points
 // Single solve: block coordinates are the grid's.
-// x passes: 3 CTAs of up to 256 threads per SM with 8 elements per thread, 2
-// with 12 (their registers); 4 for the FP32 divergence pass (64 registers,
+// x passes: the threads of 3 CTAs of 256 per SM with 8 elements per thread, of 2
+// with 12 (their registers); of 4 for the FP32 divergence pass (64 registers,
 // no spill: 0.469 -> 0.446 ms at 512^3 on B200).
+template <int N, class T> __host__ __device__ constexpr int x_min_blocks(int of256) {
+  return of256 * 256 / XCfg<N, T>::NT;
+}
 template <int N, int MODE, class T> __host__ __device__ constexpr int xfwd_min_blocks() {
-  return reg_elems(N) == 8 ? (sizeof(T) == 4 && MODE != 2 ? 4 : 3) : 2;
+  return x_min_blocks<N, T>(reg_elems(N) == 8 ? (sizeof(T) == 4 && MODE != 2 ? 4 : 3) : 2);
+}
+template <int N, class T> __host__ __device__ constexpr int xinv_min_blocks() {
+  return x_min_blocks<N, T>(reg_elems(N) == 8 ? 3 : 2);
 }
 template <int N, int MODE, class T>
-__global__ void __launch_bounds__(256, xfwd_min_blocks<N, MODE, T>()) xfwd_kernel(const T* __restrict__ us, const T* __restrict__ vs,
+__global__ void __launch_bounds__(XCfg<N, T>::NT, xfwd_min_blocks<N, MODE, T>()) xfwd_kernel(const T* __restrict__ us, const T* __restrict__ vs,
                                                   const T* __restrict__ ws, const T* __restrict__ rhs,
                                                   const T* __restrict__ p0, typename C2<T>::t* __restrict__ spec,
                                                   const typename C2<T>::t* __restrict__ tw,
@@ -747,7 +760,7 @@ __global__ void __launch_bounds__(256, xfwd_min_blocks<N, MODE, T>()) xfwd_kerne
   xfwd_reg_body<N, MODE, T>(us, vs, ws, rhs, p0, spec, tw, ctrl, cdiv, ddxi, blockIdx.x, blockIdx.y);
 }
 template <int N, class T, bool DEP = false>
-__global__ void __launch_bounds__(256, reg_elems(N) == 8 ? 3 : 2) xinv_kernel(const typename C2<T>::t* __restrict__ spec, T* __restrict__ p,
+__global__ void __launch_bounds__(XCfg<N, T>::NT, xinv_min_blocks<N, T>()) xinv_kernel(const typename C2<T>::t* __restrict__ spec, T* __restrict__ p,
                                                   const typename C2<T>::t* __restrict__ tw,
                                                   const Ctrl* __restrict__ ctrl) {
   if (DEP) dep_begin();
@@ -757,7 +770,7 @@ __global__ void __launch_bounds__(256, reg_elems(N) == 8 ? 3 : 2) xinv_kernel(co
 // Batched over the slots of a served ensemble: grid y = slot * N + plane.
 // `which` selects the slot's first (0) or correction (1) solve.
 template <int N, int MODE, class T>
-__global__ void __launch_bounds__(256, xfwd_min_blocks<N, MODE, T>()) xfwd_kernel_b(const SlotArgs<T>* __restrict__ slots, int which) {
+__global__ void __launch_bounds__(XCfg<N, T>::NT, xfwd_min_blocks<N, MODE, T>()) xfwd_kernel_b(const SlotArgs<T>* __restrict__ slots, int which) {
   const int sl = blockIdx.y / N;
   if (!slots[sl].active) return;
   const PoissonArgs<T>& a = which ? slots[sl].pr : slots[sl].po;
@@ -765,7 +778,7 @@ __global__ void __launch_bounds__(256, xfwd_min_blocks<N, MODE, T>()) xfwd_kerne
                             blockIdx.y - sl * N);
 }
 template <int N, class T>
-__global__ void __launch_bounds__(256, reg_elems(N) == 8 ? 3 : 2) xinv_kernel_b(const SlotArgs<T>* __restrict__ slots, int which) {
+__global__ void __launch_bounds__(XCfg<N, T>::NT, xinv_min_blocks<N, T>()) xinv_kernel_b(const SlotArgs<T>* __restrict__ slots, int which) {
   const int sl = blockIdx.y / N;
   if (!slots[sl].active) return;
   const PoissonArgs<T>& a = which ? slots[sl].pr : slots[sl].po;
