@@ -39,6 +39,15 @@ __device__ __forceinline__ size_t gidx(int i, int j, int k, int n) {
   return (size_t)i + (size_t)n * ((size_t)j + (size_t)n * (size_t)k);
 }
 
+// Whether the simulation has stopped on an error, decided once for the whole
+// CTA (a barrier; every thread calls it).  A CTA of the same launch may set
+// the status meanwhile (a wait that gave up), so threads that each read it for
+// themselves could disagree: one would leave without arming the slot barriers
+// that the others then wait on.
+__device__ __forceinline__ bool stopped(const Ctrl* ctrl) {
+  return __syncthreads_or(threadIdx.x == 0 && ctrl->status != 0) != 0;
+}
+
 // ---- dependent launches ----
 // First in every kernel that launch_dep may launch: lets the next kernel's
 // CTAs be scheduled once every CTA of this one is here, and returns when the

@@ -216,7 +216,6 @@ __device__ __forceinline__ void rcol_run(int total, const typename C2<T>::t* __r
       mbar_init(bar, 1);
       mbar_init_fence();
     }
-    __syncthreads();
   }
   unsigned phase = 0;
   bool pend = false;  // a box load of the next slab is in flight (the same in every thread)
@@ -259,9 +258,14 @@ __device__ __forceinline__ void rcol_run(int total, const typename C2<T>::t* __r
       cp_async_commit();
     }
   };
+  // Thread 0, which arms the barrier and issues the boxes, decides for the CTA
+  // whether a slab is live (see stopped() for why); the barrier it takes is one
+  // the loop needs anyway.
+  const auto agree = [](bool live) { return __syncthreads_and(threadIdx.x != 0 || live) != 0; };
   ColSlab nx;
   if constexpr (PF) {
     nx = get(blockIdx.x);
+    if constexpr (TMA) nx.live = agree(nx.live);  // also publishes the slot barrier
     prefetch(nx);
   }
   for (int it = blockIdx.x; it < total; it += gridDim.x) {
@@ -284,7 +288,7 @@ __device__ __forceinline__ void rcol_run(int total, const typename C2<T>::t* __r
       }
       nx.live = false;
       if (it + (int)gridDim.x < total) nx = get(it + gridDim.x);
-      if constexpr (TMA) __syncthreads();  // every thread has read the buffer the next box fills
+      if constexpr (TMA) nx.live = agree(nx.live);  // every thread has read the buffer the next box fills
       prefetch(nx);
       if (!sl.live) continue;
     } else {

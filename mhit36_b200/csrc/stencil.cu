@@ -281,7 +281,6 @@ template <class T, bool SLOT>
 __device__ __forceinline__ void phase_body(const StencilArgs<T>& a, const T* __restrict__ phi_in,
                                            T* __restrict__ phi_out, int nz, int bx, int by, int bz,
                                            const PhaseMaps* __restrict__ maps) {
-  if (a.ctrl->status) return;
   constexpr int TY = PTY, NT = PNT;
   typedef PhaseGeo<T> G;
   constexpr int LX = TX + 4, PE = LX * G::EY, EX = G::EX, OFF = G::XS - 2, SL = G::PSL;
@@ -311,7 +310,7 @@ __device__ __forceinline__ void phase_body(const StencilArgs<T>& a, const T* __r
       tensormap_acquire(&maps->w);
     }
   }
-  __syncthreads();
+  if (stopped(a.ctrl)) return;  // also publishes the barriers and the table
   const T eps = (T)a.c.eps, enumv = (T)a.c.enumv, tiny = (T)a.c.tiny;
   const T dt = (T)a.c.dt, hdxi = (T)(0.5 * a.c.dxi);
   const double gamma = 1.0 * a.ctrl->gumax;  // multi/main.f90:362
@@ -531,7 +530,6 @@ __device__ __forceinline__ void phase_body(const StencilArgs<T>& a, const T* __r
 template <class T, bool PF, int MTYv, bool TMA>
 __device__ __forceinline__ void momentum_body(const StencilArgs<T>& a, int nz, int bx, int by, int bz,
                                               const PlaneMaps* __restrict__ maps, bool gmaps) {
-  if (a.ctrl->status) return;
   // MPT output rows per thread (rows ty + 8h): 256 threads for either tile
   constexpr int TY = MTYv, MPT = MTYv / 8, NT = TX * 8;
   typedef MomGeo<T, MTYv> G;
@@ -597,20 +595,18 @@ __device__ __forceinline__ void momentum_body(const StencilArgs<T>& a, int nz, i
 #pragma unroll
   for (int q2 = 0; q2 < NS; ++q2) sl[q2] = q2;
   unsigned bar_phase = 0;  // bit s: parity of the next phase of slot s's barrier
-  if (tma) {
-    if (tid == 0) {
+  if (tma && tid == 0) {
 #pragma unroll
-      for (int q2 = 0; q2 < NS; ++q2) mbar_init(s_bar + q2, 1);
-      mbar_init_fence();
-      if (gmaps) {  // maps in the ensemble's slot table
-        tensormap_acquire(&maps->u);
-        tensormap_acquire(&maps->v);
-        tensormap_acquire(&maps->w);
-        if (PF) tensormap_acquire(&maps->phi);
-      }
+    for (int q2 = 0; q2 < NS; ++q2) mbar_init(s_bar + q2, 1);
+    mbar_init_fence();
+    if (gmaps) {  // maps in the ensemble's slot table
+      tensormap_acquire(&maps->u);
+      tensormap_acquire(&maps->v);
+      tensormap_acquire(&maps->w);
+      if (PF) tensormap_acquire(&maps->phi);
     }
-    __syncthreads();
   }
+  if (stopped(a.ctrl)) return;  // also publishes the barriers
 
   // Plane m of u, v, w (1-cell ring) and phi (2-cell ring) is copied into a
   // ring slot PD iterations ahead of its use, so the HBM latency of the
