@@ -117,11 +117,11 @@ template <int DIR, class C> struct DFT<12, DIR, C> {
 // the canonical positions themselves (NS*R = N makes them x[j + r*N/R]), so
 // they stay in registers.
 //
-// R12 takes one stage and one exchange out of the column passes, which are
-// bound by their shared-memory exchanges (384^3 FP64 on B200: z solve 388 ->
-// 346 us, y passes 223 -> 214; 192^3: 46 -> 41 and 31 -> 28).  The x passes go
-// without it: their lines follow one another in shared memory, and writes 12
-// elements apart conflict there (384^3: x inverse 225 -> 276 us).
+// R12 takes one stage and one exchange out of the column passes up to 384^3,
+// which are bound by their shared-memory exchanges (384^3 FP64 on B200: z solve
+// 389 -> 345 us, y passes 223 -> 215; the other sizes where the rule stands).
+// The x passes go without it: their lines follow one another in shared memory,
+// and writes 12 elements apart conflict there (384^3: x inverse 225 -> 276 us).
 //
 // Exchange buffer: `at(n)` is the shared-memory slot of element n of the
 // thread's line.  The exchanges write either consecutive elements or

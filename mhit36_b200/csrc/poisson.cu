@@ -178,6 +178,14 @@ template <int N, class T> struct RCfg {
   // with the prefetch, and its served stream ran 28% slower)
   static constexpr bool pf_batched(int) { return sizeof(T) == 8; }
   static constexpr bool stw(int) { return true; }
+  // Sizes 3*2^k: a radix-12 first stage up to 384.  At 768 it spills more than
+  // the stage it saves is worth.  B200, radix 4 first -> radix 12 first, us:
+  //   y pass: 192^3 FP64 31 -> 28, FP32 20 -> 18; 384^3 FP64 223 -> 215, FP32 126
+  //   -> 121; 768^3 FP64 2780 -> 4120, FP32 1130 -> 1240; 96^3 equal
+  //   z solve: 192^3 47 -> 41, 35 -> 31; 384^3 389 -> 345, 226 -> 204; 768^3 5480
+  //   -> 5690, 2390 -> 2440
+  // The batched passes follow (192^3 y 35 -> 34 and 19 -> 17, z 55 -> 49 and 37 -> 35).
+  static constexpr bool R12 = N <= 384;
   // (12 elements per thread: y passes 128 in FP64 and 80 in FP32, z solves
   // 168 and 128.)
   static constexpr int minb(int kind) {
@@ -203,6 +211,7 @@ template <int N, int KIND, class T, bool PF, bool TMA, class Getter>
 __device__ __forceinline__ void rcol_run(int total, const typename C2<T>::t* __restrict__ gtw, Getter get) {
   typedef typename C2<T>::t C;
   constexpr int CC = RCfg<N, T>::CC, E = RCfg<N, T>::E, TPC = N / E;
+  constexpr bool R12 = RCfg<N, T>::R12;
   extern __shared__ __align__(128) unsigned char smem_raw[];
   constexpr int NT = RCfg<N, T>::NT;
   C* s = reinterpret_cast<C*>(smem_raw);
@@ -300,14 +309,14 @@ __device__ __forceinline__ void rcol_run(int total, const typename C2<T>::t* __r
     }
     C* col = static_cast<C*>(sl.spec) + c;
     if (KIND == 0) {
-      reg_fft_stages<N, 1, -1, true>(v, s, tw, t, at);
+      reg_fft_stages<N, 1, -1, R12>(v, s, tw, t, at);
     } else if (KIND == 1) {
-      reg_fft_stages<N, 1, +1, true>(v, s, tw, t, at);
+      reg_fft_stages<N, 1, +1, R12>(v, s, tw, t, at);
     } else {
       // forward z FFT, then -psi/k2/(nx*ny*nz) per mode (multi/main.f90:792,
       // one reciprocal per mode; mode (0,0,0) and the pitch padding beyond
       // kx = N/2 set to 0), then the inverse z FFT
-      reg_fft_stages<N, 1, -1, true>(v, s, tw, t, at);
+      reg_fft_stages<N, 1, -1, R12>(v, s, tw, t, at);
       const double nnn = (double)((long long)N * (long long)N * (long long)N);
       const double* k2tab = sl.k2tab;
       const int mx = sl.m0 + c, jy = sl.jy;
@@ -325,7 +334,7 @@ __device__ __forceinline__ void rcol_run(int total, const typename C2<T>::t* __r
           v[m].y = v[m].y * f;
         }
       }
-      reg_fft_stages<N, 1, +1, true>(v, s, tw, t, at);
+      reg_fft_stages<N, 1, +1, R12>(v, s, tw, t, at);
     }
 #pragma unroll
     for (int m = 0; m < E; ++m) col[(size_t)(t + TPC * m) * sl.stride] = v[m];
