@@ -48,6 +48,9 @@ __device__ __forceinline__ bool stopped(const Ctrl* ctrl) {
   return __syncthreads_or(threadIdx.x == 0 && ctrl->status != 0) != 0;
 }
 
+// The larger of two values, NaN if either is (fmax drops a NaN).
+__device__ __forceinline__ double max_nan(double a, double b) { return (a > b || a != a) ? a : b; }
+
 // ---- dependent launches ----
 // First in every kernel that launch_dep may launch: lets the next kernel's
 // CTAs be scheduled once every CTA of this one is here, and returns when the

@@ -39,6 +39,7 @@ __global__ void __launch_bounds__(DNT, 3) stats_kernel(const T* __restrict__ u, 
   const int k0 = blockIdx.z * kz;
   const double h = 0.5 * dxi_d;
   double s[NSTAT] = {0, 0, 0, 0, INFINITY, -INFINITY, 0, 0};
+  bool bad = false;  // a NaN was seen, which fmax drops
   const size_t zb = nn * (size_t)wrapi(k0 - 1, n), zc = nn * (size_t)k0;
   double um = (double)u[zb + oc] - mu, vm = (double)v[zb + oc] - mv, wm = (double)w[zb + oc] - mw;
   double uc = (double)u[zc + oc] - mu, vc = (double)v[zc + oc] - mv, wc = (double)w[zc + oc] - mw;
@@ -66,7 +67,7 @@ __global__ void __launch_bounds__(DNT, 3) stats_kernel(const T* __restrict__ u, 
     // forward-difference divergence of the projection (multi/main.f90:723-725)
     const double div = ((uxp - uc) + (vyp - vc) + (wzp - wc)) * dxi_c;
     s[2] = fmax(s[2], fabs(div));
-    if (div != div) s[2] = NAN;
+    bad |= div != div;
     if (phi) {
       const double f = (double)lf;
       s[3] += f;
@@ -77,12 +78,14 @@ __global__ void __launch_bounds__(DNT, 3) stats_kernel(const T* __restrict__ u, 
     vm = vc; vc = vzp;
     wm = wc; wc = wzp;
   }
+  if (bad) s[2] = NAN;
   __shared__ double red[DNT / 32][NSTAT];
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) {
     for (int t = 0; t < NSTAT; ++t) {
       const double x = __shfl_xor_sync(0xffffffffu, s[t], o);
-      if (t == 2 || t == 5) s[t] = fmax(s[t], x);
+      if (t == 2) s[t] = max_nan(s[t], x);
+      else if (t == 5) s[t] = fmax(s[t], x);
       else if (t == 4) s[t] = fmin(s[t], x);
       else s[t] += x;
     }
@@ -94,7 +97,8 @@ __global__ void __launch_bounds__(DNT, 3) stats_kernel(const T* __restrict__ u, 
     for (int wdx = 1; wdx < DNT / 32; ++wdx)
       for (int t = 0; t < NSTAT; ++t) {
         const double x = red[wdx][t];
-        if (t == 2 || t == 5) red[0][t] = fmax(red[0][t], x);
+        if (t == 2) red[0][t] = max_nan(red[0][t], x);
+        else if (t == 5) red[0][t] = fmax(red[0][t], x);
         else if (t == 4) red[0][t] = fmin(red[0][t], x);
         else red[0][t] += x;
       }
@@ -109,7 +113,8 @@ __global__ void stats_final_kernel(const double* __restrict__ partials, int npar
   for (int b = threadIdx.x; b < nparts; b += 256)
     for (int t = 0; t < NSTAT; ++t) {
       const double x = partials[(size_t)b * NSTAT + t];
-      if (t == 2 || t == 5) s[t] = fmax(s[t], x);
+      if (t == 2) s[t] = max_nan(s[t], x);
+      else if (t == 5) s[t] = fmax(s[t], x);
       else if (t == 4) s[t] = fmin(s[t], x);
       else s[t] += x;
     }
@@ -120,7 +125,8 @@ __global__ void stats_final_kernel(const double* __restrict__ partials, int npar
       for (int t = 0; t < NSTAT; ++t) {
         const double x = red[threadIdx.x + st][t];
         double& y = red[threadIdx.x][t];
-        if (t == 2 || t == 5) y = fmax(y, x);
+        if (t == 2) y = max_nan(y, x);
+        else if (t == 5) y = fmax(y, x);
         else if (t == 4) y = fmin(y, x);
         else y += x;
       }

@@ -915,8 +915,7 @@ __device__ __forceinline__ void project_refine_body(const StencilArgs<float>& a,
     const double v1 = (double)a.vs[gyp] - dtr * (P(gyp) - pc) * dxi;
     const double w1 = wsn - dtr * (pn - pc) * dxi;
     const double div = ((u1 - uo) + (v1 - vo) + (w1 - wo)) * dxi;
-    mdiv = fmax(mdiv, fabs(div));
-    if (div != div) mdiv = NAN;
+    mdiv = max_nan(mdiv, fabs(div));
     a.uo[g] = (float)uo;
     a.vo[g] = (float)vo;
     a.wo[g] = (float)wo;
@@ -937,7 +936,8 @@ __device__ __forceinline__ void project_refine_body(const StencilArgs<float>& a,
 #pragma unroll
     for (int t = 0; t < 3; ++t) vals[t] += __shfl_xor_sync(0xffffffffu, vals[t], o);
 #pragma unroll
-    for (int t = 3; t < 7; ++t) vals[t] = fmax(vals[t], __shfl_xor_sync(0xffffffffu, vals[t], o));
+    for (int t = 3; t < 6; ++t) vals[t] = fmax(vals[t], __shfl_xor_sync(0xffffffffu, vals[t], o));
+    vals[6] = max_nan(vals[6], __shfl_xor_sync(0xffffffffu, vals[6], o));
   }
   __shared__ double red[NT / 32][7];
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
@@ -949,7 +949,8 @@ __device__ __forceinline__ void project_refine_body(const StencilArgs<float>& a,
     for (int t = 0; t < 7; ++t) r[t] = red[0][t];
     for (int w = 1; w < NT / 32; ++w) {
       for (int t = 0; t < 3; ++t) r[t] += red[w][t];
-      for (int t = 3; t < 7; ++t) r[t] = fmax(r[t], red[w][t]);
+      for (int t = 3; t < 6; ++t) r[t] = fmax(r[t], red[w][t]);
+      r[6] = max_nan(r[6], red[w][6]);
     }
     const size_t b = (size_t)bx + (size_t)gx * (by + (size_t)gy * bz);
     for (int t = 0; t < 7; ++t) a.partials[b * 7 + t] = r[t];
@@ -1016,16 +1017,12 @@ __global__ void __launch_bounds__(NT) refine_div_kernel(StencilArgs<float> a, co
     const double v1 = vsy - dtr * (s[cell + PX] - pc) * dxi;
     const double w1 = wsn - dtr * (pn - pc) * dxi;
     const double div = ((u1 - uo) + (v1 - vo) + (w1 - wo)) * dxi;
-    mdiv = fmax(mdiv, fabs(div));
-    if (div != div) mdiv = NAN;
+    mdiv = max_nan(mdiv, fabs(div));
     pm = pc;
     pc = pn;
     wsc = wsn;
   }
-  for (int o = 16; o > 0; o >>= 1) {
-    const double x = __shfl_xor_sync(0xffffffffu, mdiv, o);
-    mdiv = (x != x) ? x : fmax(mdiv, x);
-  }
+  for (int o = 16; o > 0; o >>= 1) mdiv = max_nan(mdiv, __shfl_xor_sync(0xffffffffu, mdiv, o));
   if ((threadIdx.x & 31) == 0) atomicMax(out, (unsigned long long)__double_as_longlong(fabs(mdiv)));
 }
 
