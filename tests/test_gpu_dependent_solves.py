@@ -58,3 +58,21 @@ def test_chained_solves(n, graph):
         torch.cuda.synchronize()
     got = buf[SOLVES & 1]
     assert float((got - want).abs().max() / want.abs().max()) <= TOL
+
+
+@pytest.mark.parametrize("n", [32, 64, 96, 128, 192])  # 192: plain launches
+def test_chained_solves_through_a_handle(n):
+    import torch
+    from mhit36_b200 import Solver
+    from mhit36_b200.config import InputParams
+    gen = torch.Generator(device="cuda").manual_seed(n)
+    rhs = torch.randn(n ** 3, dtype=torch.float64, device="cuda", generator=gen)
+    want = _chain(rhs, n)
+    buf = [rhs.clone(), torch.empty_like(rhs)]
+    torch.cuda.synchronize()
+    with Solver(n, InputParams(grid_mode=1), phase_field=False) as s:
+        for q in range(SOLVES):
+            s.poisson_device(buf[q & 1].data_ptr(), buf[(q & 1) ^ 1].data_ptr())
+        torch.cuda.synchronize()
+    got = buf[SOLVES & 1]
+    assert float((got - want).abs().max() / want.abs().max()) <= TOL
