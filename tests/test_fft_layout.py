@@ -36,6 +36,10 @@ def lines_per_cta(n):
     return 8 if n <= 256 else (4 if n <= 512 else 2)
 
 
+def x_pairs_per_cta(n):  # the x passes' own CTAs
+    return lines_per_cta(n) // 2 if 192 <= n <= 512 else lines_per_cta(n)
+
+
 def reg_rows(n):
     return n + n // 8
 
@@ -118,14 +122,15 @@ def test_column_slab_layout(n, elem):
 
 @pytest.mark.parametrize("n", SIZES)
 def test_x_line_layouts(n):
-    """x passes: FP64 lines at c*reg_rows(N) + pad(n), FP32 lines at
-    c*N + swz(n); the fused x inverse + projection (n >= 256) adds one halo
+    """x passes (P line pairs, half a column chunk from 192 to 512): FP64 lines
+    at c*reg_rows(N) + pad(n), FP32 lines at c*N + swz(n); the fused x inverse + projection (n >= 256) adds one halo
     pair, P + 1 lines at c*reg_rows(N) + pad(n)."""
-    p = lines_per_cta(n)
+    p = x_pairs_per_cta(n)
     rng = np.random.default_rng(n)
     cases = [(p, lambda c, k: c * reg_rows(n) + pad(k), p * reg_rows(n)),
              (p, lambda c, k: c * n + swz(k), p * n)]
     if n >= 256:
+        p = lines_per_cta(n)
         cases.append((p + 1, lambda c, k: c * reg_rows(n) + pad(k), (p + 1) * reg_rows(n)))
     for nlines, at, nslots in cases:
         x = rng.standard_normal((nlines, n)) + 1j * rng.standard_normal((nlines, n))

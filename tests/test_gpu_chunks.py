@@ -1,6 +1,7 @@
-"""The stencil kernels' default z chunks on small grids: uneven chunks (n not
-a multiple of their number) and chunks of a few planes give the same bits as
-the even 32-plane chunks, in both forms and with and without the phase field."""
+"""The stencil kernels' default z chunks: uneven chunks (n not a multiple of
+their number; the FP32 phase kernel takes them up to 256^3) and chunks of a few
+planes give the same bits as the even 32-plane chunks, in both forms and with
+and without the phase field."""
 import numpy as np
 import pytest
 
@@ -9,7 +10,7 @@ pytestmark = pytest.mark.gpu
 
 @pytest.mark.parametrize("n,precision,phase", [(32, "fp64", True), (64, "fp64", False), (96, "fp64", True),
                                                (128, "fp64", True), (192, "fp64", True), (96, "fp32", True),
-                                               (192, "fp32", True)])
+                                               (192, "fp32", True), (256, "fp32", True)])
 def test_default_chunks_match_even_chunks(n, precision, phase):
     from mhit36_b200 import Solver, fields
     from mhit36_b200.config import InputParams

@@ -25,6 +25,28 @@ def test_second_batch_on_the_same_ensemble():
                 ens.release(i)
 
 
+def test_batch_after_cancelled_requests():
+    """Cancelled while queued, while loading or running, and when done (which
+    leaves a request as it is): the next batch's results are its own."""
+    from mhit36_b200.ensemble import Ensemble
+    with Ensemble(slots_per_class=2) as ens:
+        for batch in range(3):
+            cases = [_case(64, True, 20 * batch + i) for i in range(4)]
+            ids = [ens.submit(64, _params(), *c, nsteps=4 if i else 5000) for i, c in enumerate(cases)]
+            for _ in range(30 * batch):  # admitted and loading, or some steps in
+                ens.progress()
+            ens.cancel(ids[0])
+            ens.cancel(ids[3])
+            gone = [i for i in (0, 3) if ens.query(ids[i])["state"] == "cancelled"]
+            assert 0 in gone
+            ens.run()
+            for i in range(4):
+                if i not in gone:
+                    _same(ens.result(ids[i]), _solo(64, _params(), cases[i], 4))
+            for i in ids:
+                ens.release(i)
+
+
 def test_large_result_is_copied_whole():
     """A field of 7 MB is copied by several threads."""
     from mhit36_b200.ensemble import Ensemble

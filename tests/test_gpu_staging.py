@@ -4,7 +4,8 @@ The phase and momentum kernels stage each z plane of their inputs in
 shared-memory rings.  Tiles whose staged boxes lie inside the grid load a
 plane with tensor-map box loads (cp.async.bulk.tensor) completed on a
 shared-memory barrier; tiles at the periodic edges copy the same boxes
-element-wise with cp.async and wrap, into the same cells.  Every grid from
+element-wise with cp.async and wrap, into the same cells (of the phase kernel
+phi only: its velocities arrive by box loads on every tile).  Every grid from
 96^3 up has both kinds of tile, so the step parity tests against the oracle
 (tests/test_gpu_parity.py, tests/test_gpu_bench_workload.py) cover both; at
 32^3 and 64^3 every tile is an edge tile.
@@ -12,9 +13,9 @@ element-wise with cp.async and wrap, into the same cells.  Every grid from
 This file tests the bounded barrier wait: with nothing arriving it gives up
 after the given number of cycles and reports MHIT_ERR_TIMEOUT, the kernel
 returns, and the CUDA context stays usable (a 96^3 step afterwards matches
-the oracle).  The served ensemble's batched kernels copy element-wise on every tile;
-tests/test_gpu_ensemble.py checks them bitwise against the solo handle at
-grids with interior tiles.
+the oracle).  The served ensemble's batched kernels stage as the solo handle's
+do, with tensor maps kept in the slot table; tests/test_gpu_ensemble.py checks
+them bitwise against the solo handle at grids with interior tiles.
 """
 import ctypes
 
