@@ -316,14 +316,18 @@ __device__ __forceinline__ void phase_body(const StencilArgs<T>& a, const T* __r
   const double gamma = 1.0 * a.ctrl->gumax;  // multi/main.f90:362
   const T gh = (T)(gamma * (0.5 * a.c.dxi)), ge = (T)(gamma * (a.c.eps * a.c.ddxi));
   const T mu = (T)a.ctrl->mean[0], mv = (T)a.ctrl->mean[1], mw = (T)a.ctrl->mean[2];
-  const T floor0 = a.c.phi_floor ? (T)0 : (T)-INFINITY;
+  const bool floored = a.c.phi_floor;
+  const T floor0 = floored ? (T)0 : (T)-INFINITY;
   const T inv12e = (T)1 / ((T)1 + (T)2 * enumv);
   // psi where min(phi,1) is exactly 1 (drop interiors) or so small that both
   // val + enum == enum and 1 - val + enum == 1 - 0 + enum in floating point
   // (far field; the first implies the second, since it needs |val| below
   // half an ulp of enum, far under 2^-54): there the reference's expression
   // evaluates to psi1 / psi0 exactly, so those constants are computed once
-  // and the log is skipped -- bitwise the same values.
+  // and the log is skipped -- bitwise the same values.  With the floor every
+  // negative phi is of the second kind.  Without it a phi at or below -enum has
+  // the logarithm of 0 (-inf) or of a negative number (NaN), which tang_log, for
+  // positive numbers only, does not give (FP32's __logf does).
   const T psi0 = eps * PsiMath<T>::log_ratio((T)0 + enumv, (T)1 - (T)0 + enumv, s_tab);
   const T psi1 = eps * PsiMath<T>::log_ratio((T)1 + enumv, (T)1 - (T)1 + enumv, s_tab);
   const size_t nn = (size_t)n * n;
@@ -405,9 +409,17 @@ __device__ __forceinline__ void phase_body(const StencilArgs<T>& a, const T* __r
     for (int r = 0; r < NPE; ++r) {
       if (r < NPE - 1 || tid + r * NT < PE) {
         const int ep = pidx(r);
-        const T val = fmax(fmin(Ph0[ep], (T)1), floor0);
-        Ps0[ep] = (val + enumv == enumv) ? psi0
-                 : ((val == (T)1) ? psi1 : eps * PsiMath<T>::log_ratio(val + enumv, (T)1 - val + enumv, s_tab));
+        const T val = fmin(Ph0[ep], (T)1), sum = val + enumv;
+        T psi;
+        if (sum <= enumv && (floored || sum == enumv)) {
+          psi = psi0;
+        } else if (val < (T)1) {
+          psi = eps * PsiMath<T>::log_ratio(sum, (T)1 - val + enumv, s_tab);
+          if (sizeof(T) == 8 && !floored && sum <= (T)0) psi = sum < (T)0 ? (T)NAN : -(T)INFINITY;
+        } else {
+          psi = psi1;
+        }
+        Ps0[ep] = psi;
       }
     }
     // psi(m) is visible and every thread is done with iteration m-1, so the
