@@ -322,7 +322,9 @@ int mhit_ens_progress(mhit_ensemble* e, int* pending);
  * mhit_ens_wait instead of spinning on mhit_ens_progress. */
 int mhit_ens_wait(mhit_ensemble* e, double timeout_s, int* ready);
 int mhit_ens_query(mhit_ensemble* e, int64_t id, mhit_ens_info* out);
-/* Final fields of a done request (keep_result = 1), raw layout float64. */
+/* Final fields of a done request (keep_result = 1), raw layout float64; of a
+ * request that stopped on a step's error, the fields it stopped with.  One
+ * whose transfer failed has none: MHIT_ERR_STATE. */
 int mhit_ens_result(mhit_ensemble* e, int64_t id, double* u, double* v, double* w, double* phi);
 int mhit_ens_release(mhit_ensemble* e, int64_t id);
 int mhit_ens_cancel(mhit_ensemble* e, int64_t id);

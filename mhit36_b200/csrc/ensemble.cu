@@ -29,7 +29,6 @@
 // There is no counterpart in the reference, which runs one simulation per job.
 #include <cuda_runtime.h>
 #include <math.h>
-#include <stdlib.h>
 #include <string.h>
 
 #include <algorithm>
@@ -46,6 +45,7 @@
 #include <vector>
 
 #include "hostcopy.h"
+#include "hostpool.h"
 #include "internal.h"
 #include "mhit.h"
 
@@ -64,80 +64,13 @@ enum { RQ_QUEUED = 0, RQ_RUNNING = 1, RQ_DONE = 2, RQ_FAILED = 3, RQ_CANCELLED =
 // progress of a request's job on a transfer thread
 enum { IO_NONE = 0, IO_QUEUED = 1, IO_DONE = 2, IO_FAILED = 3 };
 
-// Host buffers for the final fields of requests.  A released request's buffers
-// are kept for the next ones (up to kMost bytes, freed with the ensemble): a
-// fresh one costs a page fault per 4 KB, half of a 96^3 request's download.
-class HostPool {
- public:
-  static constexpr size_t kMost = (size_t)512 << 20;
-  double* take(size_t count) {
-    {
-      std::lock_guard<std::mutex> g(mu_);
-      auto it = free_.find(count);
-      if (it != free_.end()) {
-        double* p = it->second;
-        free_.erase(it);
-        kept_ -= count * sizeof(double);
-        return p;
-      }
-    }
-    return static_cast<double*>(malloc(count * sizeof(double)));
-  }
-  void give(double* p, size_t count) {
-    if (!p) return;
-    {
-      std::lock_guard<std::mutex> g(mu_);
-      if (kept_ + count * sizeof(double) <= kMost) {
-        try {
-          free_.emplace(count, p);
-          kept_ += count * sizeof(double);
-          return;
-        } catch (...) {  // no room for the entry: the buffer is freed
-        }
-      }
-    }
-    free(p);
-  }
-  ~HostPool() {
-    for (auto& b : free_) free(b.second);
-  }
-
- private:
-  std::mutex mu_;
-  std::multimap<size_t, double*> free_;
-  size_t kept_ = 0;
-};
-
-// A buffer of the pool, given back with its request.
-struct HostBuf {
-  HostPool* pool = nullptr;
-  double* p = nullptr;
-  size_t count = 0;
-  bool take(HostPool* from, size_t n) {
-    drop();
-    pool = from;
-    p = from->take(n);
-    count = p ? n : 0;
-    return p != nullptr;
-  }
-  void drop() {
-    if (p) pool->give(p, count);
-    p = nullptr;
-    count = 0;
-  }
-  HostBuf() = default;
-  HostBuf(const HostBuf&) = delete;
-  HostBuf& operator=(const HostBuf&) = delete;
-  ~HostBuf() { drop(); }
-};
-
 struct Request {
   int64_t id = 0;
   int n = 0, pf = 0, precision = 0, nsteps = 0, keep = 1, borrow = 0;
   mhit_params prm;
   std::vector<double> in[4];          // owned copies of the inputs (not borrowed), dropped after upload
   const double* src[4] = {nullptr, nullptr, nullptr, nullptr};  // what the upload reads
-  HostBuf out[4];                     // final fields when keep = 1
+  mhit::ResultFields out;             // final fields when keep = 1
   Ctrl fin;                           // final control block (downloaded)
   int state = RQ_QUEUED;
   int cls = -1, slot = -1;
@@ -206,7 +139,7 @@ class Transfer {
   static constexpr size_t kChunk = (size_t)32 << 20;  // bytes per staging chunk
   static constexpr size_t kSmall = (size_t)64 << 10;  // tables and control block
 
-  cudaError_t start(int device, HostPool* pool) {
+  cudaError_t start(int device, mhit::HostPool* pool) {
     device_ = device;
     pool_ = pool;
     cudaError_t e;
@@ -355,7 +288,7 @@ class Transfer {
   cudaError_t download(const Job& j, std::string* where);
 
   int device_ = 0;
-  HostPool* pool_ = nullptr;
+  mhit::HostPool* pool_ = nullptr;
   cudaStream_t st_ = nullptr;
   void* stage_[2] = {nullptr, nullptr};
   cudaEvent_t sev_[2] = {nullptr, nullptr};
@@ -377,7 +310,7 @@ struct mhit_ensemble {
   int slots_per_class = 8;
   int64_t next_id = 1;
   double t0 = 0;
-  HostPool pool;  // outlives the requests and the transfer threads
+  mhit::HostPool pool;  // outlives the requests and the transfer threads
   std::map<int64_t, std::unique_ptr<Request>> reqs;
   std::deque<int64_t> queue;
   std::vector<std::unique_ptr<Class>> classes;
@@ -785,10 +718,8 @@ cudaError_t Transfer::download(const Job& j, std::string* where) {
   if (r->keep) {
     const void* src[4] = {b.f[0], b.f[1], b.f[2], b.f[13]};
     const int nf = c->pf ? 4 : 3;
-    for (int f = 0; f < nf; ++f) {
-      TCK(r->out[f].take(pool_, N3) ? cudaSuccess : cudaErrorMemoryAllocation);
-      TCK(get(r->out[f].p, src[f], N3, el));
-    }
+    TCK(r->out.fill(pool_, nf, N3, cudaErrorMemoryAllocation,
+                    [&](double* dst, int f) { return get(dst, src[f], N3, el); }));
   }
   return cudaSuccess;
 }
@@ -1241,12 +1172,12 @@ int mhit_ens_result(mhit_ensemble* e, int64_t id, double* u, double* v, double* 
   if (it == e->reqs.end()) return MHIT_ERR_INVALID;
   Request* r = it->second.get();
   if (r->state != RQ_DONE && r->state != RQ_FAILED) return MHIT_ERR_STATE;
-  if (!r->keep || !r->out[0].p) return MHIT_ERR_STATE;
+  if (!r->keep || !r->out.held()) return MHIT_ERR_STATE;
   double* dst[4] = {u, v, w, phi};
   for (int f = 0; f < 4; ++f)
-    if (dst[f] && r->out[f].p) {
-      const size_t b = r->out[f].count * sizeof(double);
-      mhit::parallel_copy(dst[f], b, r->out[f].p, b, b, 1);
+    if (dst[f] && r->out.field(f)) {
+      const size_t b = r->out.count() * sizeof(double);
+      mhit::parallel_copy(dst[f], b, r->out.field(f), b, b, 1);
     }
   return MHIT_OK;
 }
