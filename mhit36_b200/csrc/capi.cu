@@ -59,7 +59,7 @@ struct mhit_handle {
   // check) is recomputed on request.
   bool dp_in_spec = false;
   bool have_step = false;     // a step ran since the fields were set (ustar, p0 are its own)
-  mhit::PinnedChunks chunks;  // for host copies of large pageable arrays (first use)
+  mhit::PinnedPieces pieces;  // for host copies of large pageable arrays (first use)
   double* stage = nullptr;    // FP32 form: device staging of FP64 planes for host copies (first use)
   double* div_out = nullptr;  // device: max |div u| of the FP64 projection (FP32 refine form)
   double* stat_partials = nullptr;
@@ -127,7 +127,7 @@ void free_all(mhit_handle* h) {
   h->allocs.clear();
   if (h->h_ctrl) cudaFreeHost(h->h_ctrl);
   if (h->h_stat) cudaFreeHost(h->h_stat);
-  h->chunks.release();
+  h->pieces.release();
   if (h->st) cudaStreamDestroy(h->st);
 }
 
@@ -289,79 +289,94 @@ size_t host_offset(int n, int layout, int k) {
 }
 size_t host_pitch(int n, int layout) { return sizeof(double) * n * (size_t)(layout == MHIT_LAYOUT_RAW ? n : n + 2); }
 
-// A field crosses the boundary in chunks of whole planes (up to 16 MB of
-// float64), in stream order: f(first plane, planes).  FP32 fields pass
-// through a device buffer of one chunk, where they are rounded / widened.
-template <class F> cudaError_t for_chunks(mhit_handle* h, bool f32, const F& f) {
-  const int n = h->n;
+// The FP32 form's device buffer, in which fields cross the boundary as float64
+// and are rounded / widened: whole planes, up to 16 MB, or all pinned pieces.
+int stage_planes(int n) {
   const size_t pb = (size_t)n * n * sizeof(double);
-  const int most = (int)std::min<size_t>(n, std::max<size_t>(1, mhit::PinnedChunks::kBytes / pb));
-  cudaError_t e;
-  if (f32 && !h->stage && (e = dalloc(h, &h->stage, pb * most))) return e;
-  for (int k = 0; k < n; k += most)
-    if ((e = f(k, std::min(most, n - k)))) return e;
-  return cudaSuccess;
+  return (int)std::min<size_t>(n, std::max<size_t>(1, ((size_t)16 << 20) / pb));
+}
+cudaError_t need_stage(mhit_handle* h) {
+  if (h->stage) return cudaSuccess;
+  const size_t pb = (size_t)h->n * h->n * sizeof(double);
+  const size_t pieces = mhit::PinnedPieces::kThreads * mhit::PinnedPieces::piece_for(pb * h->n);
+  return dalloc(h, &h->stage, std::max(pb * stage_planes(h->n), std::min(pb * h->n, pieces)));
 }
 
-// host float64 (layout) -> device field.
+// host float64 (layout) -> device field, in stream order: a large pageable
+// array in pieces by several threads, another in one copy (FP32: in copies of
+// whole planes).
 cudaError_t put_field(mhit_handle* h, DevField d, const double* src, int layout) {
   const int n = h->n;
   const size_t plane = (size_t)n * n, pb = plane * sizeof(double), pitch = host_pitch(n, layout);
-  const bool chunks = mhit::wants_chunks(src, pb * n) && h->chunks.ready();
   cudaError_t e;
-  int b = 0;
-  return for_chunks(h, d.f32, [&](int k, int planes) -> cudaError_t {
-    double* const to = d.f32 ? h->stage : static_cast<double*>(d.ptr) + plane * k;
-    const double* from = src + host_offset(n, layout, k);
-    size_t fp = pitch;
-    if (chunks) {
-      if ((e = cudaEventSynchronize(h->chunks.ev[b]))) return e;  // the chunk's previous copy has left it
-      mhit::parallel_copy(h->chunks.buf[b], pb, from, pitch, pb, planes);
-      from = static_cast<const double*>(h->chunks.buf[b]);
-      fp = pb;
-    }
-    if ((e = cudaMemcpy2DAsync(to, pb, from, fp, pb, planes, cudaMemcpyHostToDevice, h->st))) return e;
-    if (chunks && (e = cudaEventRecord(h->chunks.ev[b], h->st))) return e;
-    b ^= 1;
-    return d.f32 ? mhit::launch_narrow(h->stage, static_cast<float*>(d.ptr) + plane * k, plane * planes, h->st)
-                 : cudaSuccess;
-  });
+  if (d.f32 && (e = need_stage(h))) return e;
+  double* const d64 = static_cast<double*>(d.ptr);
+  float* const d32 = static_cast<float*>(d.ptr);
+  if (mhit::wants_pieces(src, pb * n) && h->pieces.ready(pb * n)) {
+    const mhit::HostRows rows{reinterpret_cast<char*>(const_cast<double*>(src + host_offset(n, layout, 0))), pb, pitch};
+    return h->pieces.run(h->device, pb * n, [&](int t, void* buf, cudaEvent_t ev, size_t at, size_t len) {
+      cudaError_t err = cudaEventSynchronize(ev);  // the buffer's previous copy has left it
+      if (err) return err;
+      rows.read(buf, at, len);
+      const size_t first = at / sizeof(double), count = len / sizeof(double);
+      double* const to = d.f32 ? h->stage + t * (h->pieces.piece() / sizeof(double)) : d64 + first;
+      if ((err = cudaMemcpyAsync(to, buf, len, cudaMemcpyHostToDevice, h->st))) return err;
+      if ((err = cudaEventRecord(ev, h->st))) return err;
+      return d.f32 ? mhit::launch_narrow(to, d32 + first, count, h->st) : cudaSuccess;
+    });
+  }
+  const int most = d.f32 ? stage_planes(n) : n;
+  for (int k = 0; k < n; k += most) {
+    const int planes = std::min(most, n - k);
+    double* const to = d.f32 ? h->stage : d64 + plane * k;
+    if ((e = cudaMemcpy2DAsync(to, pb, src + host_offset(n, layout, k), pitch, pb, planes, cudaMemcpyHostToDevice,
+                               h->st)))
+      return e;
+    if (d.f32 && (e = mhit::launch_narrow(h->stage, d32 + plane * k, plane * planes, h->st))) return e;
+  }
+  return cudaSuccess;
 }
 
 // device field -> host float64 (layout); FP32 fields with `add`, if given, added in FP64.
 cudaError_t get_field(mhit_handle* h, double* dst, DevField d, int layout, const float* add = nullptr) {
   const int n = h->n;
   const size_t plane = (size_t)n * n, pb = plane * sizeof(double), pitch = host_pitch(n, layout);
-  const bool chunks = mhit::wants_chunks(dst, pb * n) && h->chunks.ready();
   cudaError_t e;
-  // the chunk on the link while the one before it is copied out
-  int b = 0, k_prev = 0, planes_prev = 0;
-  auto drain = [&]() -> cudaError_t {
-    if (!planes_prev) return cudaSuccess;
-    if ((e = cudaEventSynchronize(h->chunks.ev[b ^ 1]))) return e;
-    mhit::parallel_copy(dst + host_offset(n, layout, k_prev), pitch, h->chunks.buf[b ^ 1], pb, pb, planes_prev);
-    return cudaSuccess;
-  };
-  e = for_chunks(h, d.f32, [&](int k, int planes) -> cudaError_t {
-    const double* from = static_cast<const double*>(d.ptr) + plane * k;
+  if (d.f32 && (e = need_stage(h))) return e;
+  const double* const d64 = static_cast<const double*>(d.ptr);
+  const float* const d32 = static_cast<const float*>(d.ptr);
+  if (mhit::wants_pieces(dst, pb * n) && h->pieces.ready(pb * n)) {
+    const mhit::HostRows rows{reinterpret_cast<char*>(dst + host_offset(n, layout, 0)), pb, pitch};
+    return h->pieces.run(h->device, pb * n, [&](int t, void* buf, cudaEvent_t ev, size_t at, size_t len) {
+      cudaError_t err;
+      const size_t first = at / sizeof(double), count = len / sizeof(double);
+      const double* from = d64 + first;
+      if (d.f32) {
+        double* const wide = h->stage + t * (h->pieces.piece() / sizeof(double));
+        if ((err = mhit::launch_widen(d32 + first, add ? add + first : nullptr, wide, count, h->st))) return err;
+        from = wide;
+      }
+      if ((err = cudaMemcpyAsync(buf, from, len, cudaMemcpyDeviceToHost, h->st))) return err;
+      if ((err = cudaEventRecord(ev, h->st))) return err;
+      if ((err = cudaEventSynchronize(ev))) return err;
+      rows.write(buf, at, len);
+      return cudaSuccess;
+    });
+  }
+  const int most = d.f32 ? stage_planes(n) : n;
+  for (int k = 0; k < n; k += most) {
+    const int planes = std::min(most, n - k);
+    const double* from = d64 + plane * k;
     if (d.f32) {
-      if ((e = mhit::launch_widen(static_cast<const float*>(d.ptr) + plane * k, add ? add + plane * k : nullptr,
-                                  h->stage, plane * planes, h->st)))
+      if ((e = mhit::launch_widen(d32 + plane * k, add ? add + plane * k : nullptr, h->stage, plane * planes, h->st)))
         return e;
       from = h->stage;
     }
-    if (!chunks)
-      return cudaMemcpy2DAsync(dst + host_offset(n, layout, k), pitch, from, pb, pb, planes, cudaMemcpyDeviceToHost,
-                               h->st);
-    if ((e = cudaMemcpyAsync(h->chunks.buf[b], from, pb * planes, cudaMemcpyDeviceToHost, h->st))) return e;
-    if ((e = cudaEventRecord(h->chunks.ev[b], h->st))) return e;
-    if ((e = drain())) return e;
-    k_prev = k;
-    planes_prev = planes;
-    b ^= 1;
-    return cudaSuccess;
-  });
-  return e ? e : (chunks ? drain() : cudaSuccess);
+    if ((e = cudaMemcpy2DAsync(dst + host_offset(n, layout, k), pitch, from, pb, pb, planes, cudaMemcpyDeviceToHost,
+                               h->st)))
+      return e;
+  }
+  return cudaSuccess;
 }
 
 bool f32(mhit_handle* h) { return h->precision == MHIT_FP32_REFINE; }

@@ -1175,10 +1175,7 @@ int mhit_ens_result(mhit_ensemble* e, int64_t id, double* u, double* v, double* 
   if (!r->keep || !r->out.held()) return MHIT_ERR_STATE;
   double* dst[4] = {u, v, w, phi};
   for (int f = 0; f < 4; ++f)
-    if (dst[f] && r->out.field(f)) {
-      const size_t b = r->out.count() * sizeof(double);
-      mhit::parallel_copy(dst[f], b, r->out.field(f), b, b, 1);
-    }
+    if (dst[f] && r->out.field(f)) mhit::parallel_copy(dst[f], r->out.field(f), r->out.count() * sizeof(double));
   return MHIT_OK;
 }
 

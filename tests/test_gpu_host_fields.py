@@ -48,3 +48,8 @@ def test_pinned_arrays(precision):
         s.get_fields_ptr(*[x.data_ptr() for x in got])
     for x, y in zip(a, got):
         assert torch.equal(y, x.float().double() if precision == "fp32" else x)
+
+
+@pytest.mark.parametrize("n,precision,layout", [(256, "fp32", 1), (384, "fp64", 0)])
+def test_round_trip_in_larger_pieces(n, precision, layout):
+    test_round_trip(n, precision, layout)
