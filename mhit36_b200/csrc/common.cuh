@@ -51,6 +51,18 @@ __device__ __forceinline__ bool stopped(const Ctrl* ctrl) {
 // The larger of two values, NaN if either is (fmax drops a NaN).
 __device__ __forceinline__ double max_nan(double a, double b) { return (a > b || a != a) ? a : b; }
 
+// A CTA's copy, in shared memory, of a slot table's arguments: a single
+// simulation reads them from its kernel parameters, and holding them in
+// registers spills.  NT threads, every one of which calls it.
+template <int NT, class A> __device__ __forceinline__ const A& shared_args(const A& src) {
+  static_assert(sizeof(A) % 4 == 0, "copied by words");
+  __shared__ alignas(A) unsigned sa[sizeof(A) / 4];
+  const unsigned* const s = reinterpret_cast<const unsigned*>(&src);
+  for (unsigned q = threadIdx.x; q < sizeof(sa) / 4; q += NT) sa[q] = s[q];
+  __syncthreads();
+  return *reinterpret_cast<const A*>(sa);
+}
+
 // ---- dependent launches ----
 // First in every kernel that launch_dep may launch: lets the next kernel's
 // CTAs be scheduled once every CTA of this one is here, and returns when the

@@ -737,7 +737,12 @@ __global__ void __launch_bounds__(XPCfg<N, T>::NT, 2) xinvproj_kernel(const type
   if constexpr (XPCfg<N, T>::ON) xinvproj_body<N, T>(spec, tw, a, blockIdx.x, blockIdx.y, gridDim.x);
 }
 // Batched: the FP64 step transforms the slot's spectrum, the FP32
-// refinement form its correction spectrum.
+// refinement form its correction spectrum.  At 256^3 in FP64 the slot's
+// arguments go through shared memory: with the loads that run ahead they no
+// longer fit the registers (168 bytes spilled).  Two slots on B200, us, before
+// the loads ran ahead -> from the table -> from shared memory: 256^3 FP64 434 ->
+// 446 -> 428, 512^3 FP64 3214 -> 2981 -> 3112, 256^3 FP32 350 -> 289 -> 296; 512^3
+// FP32 2505 -> 2083 -> 1976.
 template <int N, class T>
 __global__ void __launch_bounds__(XPCfg<N, T>::NT, 2) xinvproj_kernel_b(const SlotArgs<T>* __restrict__ slots,
                                                                         int zch) {
@@ -745,7 +750,11 @@ __global__ void __launch_bounds__(XPCfg<N, T>::NT, 2) xinvproj_kernel_b(const Sl
     const int sl = blockIdx.y / zch;
     if (!slots[sl].active) return;
     const PoissonArgs<T>& pa = (sizeof(T) == 4) ? slots[sl].pr : slots[sl].po;
-    xinvproj_body<N, T>(pa.spec, pa.tw, slots[sl].st, blockIdx.x, blockIdx.y - sl * zch, gridDim.x);
+    if constexpr (sizeof(T) == 8 && N <= 256)
+      xinvproj_body<N, T>(pa.spec, pa.tw, shared_args<XPCfg<N, T>::NT>(slots[sl].st), blockIdx.x,
+                          blockIdx.y - sl * zch, gridDim.x);
+    else
+      xinvproj_body<N, T>(pa.spec, pa.tw, slots[sl].st, blockIdx.x, blockIdx.y - sl * zch, gridDim.x);
   }
 }
 

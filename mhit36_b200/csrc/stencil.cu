@@ -1085,15 +1085,7 @@ template <class T>
 __global__ void __launch_bounds__(PNT, phase_min_blocks<T>()) phase_kernel_b(const SlotArgs<T>* __restrict__ slots, int zch) {
   const int sl = blockIdx.z / zch;
   if (!slots[sl].active) return;
-  // The slot's arguments are copied to shared memory once per CTA: the single
-  // simulation reads them from its kernel parameters, and holding them in
-  // registers spills.
-  __shared__ alignas(StencilArgs<T>) unsigned sa[sizeof(StencilArgs<T>) / 4];
-  static_assert(sizeof(StencilArgs<T>) % 4 == 0, "copied by words");
-  const unsigned* const src = reinterpret_cast<const unsigned*>(&slots[sl].st);
-  for (unsigned q = threadIdx.x; q < sizeof(sa) / 4; q += PNT) sa[q] = src[q];
-  __syncthreads();
-  const StencilArgs<T>& a = *reinterpret_cast<const StencilArgs<T>*>(sa);
+  const StencilArgs<T>& a = shared_args<PNT>(slots[sl].st);
   const int par = (int)(a.ctrl->nstep & 1);
   phase_body<T, true>(a, slots[sl].phi[par], slots[sl].phi[par ^ 1], zch, blockIdx.x, blockIdx.y,
                       blockIdx.z - sl * zch, &slots[sl].maps.phase[par]);
