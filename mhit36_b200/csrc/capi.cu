@@ -210,7 +210,7 @@ std::vector<Stage> step_stages(mhit_handle* h, int cur) {
     if (fused)
       v.push_back({"xinvproj", [pa, a, n, st] { return mhit::launch_xinv_project(n, pa, a, st); }});
     else
-      v.push_back({"project", [a, st] { return mhit::launch_project<double>(a, st); }});
+      v.push_back({"project", [a, st] { return mhit::launch_project(a, st); }});
   } else {
     mhit::StencilArgs<float> a = stencil_args<float>(h, cur);
     mhit::StencilArgs<float> am = a;

@@ -816,45 +816,45 @@ __device__ __forceinline__ void momentum_body(const StencilArgs<T>& a, int nz, i
 // ============================================================ projection
 // C2 + R1 (multi/main.f90:873-903): u = ustar - dt/rho*(p - p_m)*dxi, with the
 // sums and maxima of the projected u, v, w reduced per CTA in FP64.
-// z planes per projection CTA: 64 where n allows (512^3: FP64 projection plus
+// z planes per projection CTA: 64 (512^3: FP64 projection plus
 // finalize 1.47 -> 1.41 ms against 16 planes, with a quarter of the partials
 // to reduce; FP32 projection 1.85 -> 1.49 ms); fewer on small grids, so that
 // they too fill the GPU (FP64: 32^3 21 -> 8 us, 64^3 42 -> 9 us, 96^3 25 -> 14
 // us, 128^3 68 -> 30 us, 192^3 92 -> 86 us).  The FP64 loop takes it as a
 // compile-time trip count (a run-time one measured 1.79 ms at 512^3).
 __host__ __device__ constexpr int project_kz(int n) {
-  return n <= 96 ? 4 : (n <= 128 ? 8 : (n <= 192 ? 16 : (n % 64 == 0 ? 64 : 32)));
+  return n <= 96 ? 4 : (n <= 128 ? 8 : (n <= 192 ? 16 : 64));
 }
 
-template <class T, int PKZ>
-__device__ __forceinline__ void project_body(const StencilArgs<T>& a, int bx, int by, int bz, int gx, int gy) {
+template <int PKZ>
+__device__ __forceinline__ void project_body(const StencilArgs<double>& a, int bx, int by, int bz, int gx, int gy) {
   if (a.ctrl->status) return;
   const int n = a.c.n;
-  const T dtr = (T)a.c.dtr, dxi = (T)a.c.dxi;
+  const double dtr = a.c.dtr, dxi = a.c.dxi;
   const int i = bx * TX + threadIdx.x % TX, j = by * TY + threadIdx.x / TX;
   const int k0 = bz * PKZ;
   const int im = i ? i - 1 : n - 1, jm = j ? j - 1 : n - 1;
   const size_t nn = (size_t)n * n;
   double su = 0, sv = 0, sw = 0;
   double xu = -INFINITY, xv = -INFINITY, xw = -INFINITY;
-  T pprev = a.p[(size_t)i + (size_t)n * j + nn * wrapi(k0 - 1, n)];
+  double pprev = a.p[(size_t)i + (size_t)n * j + nn * wrapi(k0 - 1, n)];
 #pragma unroll 4
   for (int k = k0; k < k0 + PKZ; ++k) {
     const size_t g = (size_t)i + (size_t)n * j + nn * k;
-    const T pc = a.p[g];
-    const T uo = a.us[g] - dtr * (pc - a.p[g - i + im]) * dxi;
-    const T vo = a.vs[g] - dtr * (pc - a.p[g + (size_t)n * jm - (size_t)n * j]) * dxi;
-    const T wo = a.ws[g] - dtr * (pc - pprev) * dxi;
+    const double pc = a.p[g];
+    const double uo = a.us[g] - dtr * (pc - a.p[g - i + im]) * dxi;
+    const double vo = a.vs[g] - dtr * (pc - a.p[g + (size_t)n * jm - (size_t)n * j]) * dxi;
+    const double wo = a.ws[g] - dtr * (pc - pprev) * dxi;
     pprev = pc;
     a.uo[g] = uo;
     a.vo[g] = vo;
     a.wo[g] = wo;
-    su += (double)uo;
-    sv += (double)vo;
-    sw += (double)wo;
-    xu = fmax(xu, (double)uo);
-    xv = fmax(xv, (double)vo);
-    xw = fmax(xw, (double)wo);
+    su += uo;
+    sv += vo;
+    sw += wo;
+    xu = fmax(xu, uo);
+    xv = fmax(xv, vo);
+    xw = fmax(xw, wo);
     // NaN must not vanish in fmax: fold it into the sums too
     if (uo != uo || vo != vo || wo != wo) su = NAN;
   }
@@ -1061,9 +1061,8 @@ __global__ void __launch_bounds__(TX * 8, momentum_min_blocks<T>(PF, MTYv))
     momentum_kernel(const __grid_constant__ StencilArgs<T> a, const __grid_constant__ PlaneMaps maps) {
   momentum_body<T, PF, MTYv, true>(a, gridDim.z, blockIdx.x, blockIdx.y, blockIdx.z, &maps, false);
 }
-template <class T, int PKZ>
-__global__ void __launch_bounds__(NT, 4) project_kernel(StencilArgs<T> a) {
-  project_body<T, PKZ>(a, blockIdx.x, blockIdx.y, blockIdx.z, gridDim.x, gridDim.y);
+template <int PKZ> __global__ void __launch_bounds__(NT, 4) project_kernel(StencilArgs<double> a) {
+  project_body<PKZ>(a, blockIdx.x, blockIdx.y, blockIdx.z, gridDim.x, gridDim.y);
 }
 __global__ void __launch_bounds__(NT) project_refine_kernel(StencilArgs<float> a, const float* __restrict__ dp) {
   project_refine_body(a, dp, blockIdx.x, blockIdx.y, blockIdx.z, gridDim.x, gridDim.y);
@@ -1100,11 +1099,11 @@ __global__ void __launch_bounds__(TX * 8, momentum_min_blocks<T>(PF, MTYv)) mome
   momentum_body<T, PF, MTYv, true>(a, zch, blockIdx.x, blockIdx.y, blockIdx.z - sl * zch,
                                    &slots[sl].maps.mom[MTYv == 16 ? 1 : 0][par], true);
 }
-template <class T, int PKZ>
-__global__ void __launch_bounds__(NT, 4) project_kernel_b(const SlotArgs<T>* __restrict__ slots, int zch) {
+template <int PKZ>
+__global__ void __launch_bounds__(NT, 4) project_kernel_b(const SlotArgs<double>* __restrict__ slots, int zch) {
   const int sl = blockIdx.z / zch;
   if (!slots[sl].active) return;
-  project_body<T, PKZ>(slots[sl].st, blockIdx.x, blockIdx.y, blockIdx.z - sl * zch, gridDim.x, gridDim.y);
+  project_body<PKZ>(slots[sl].st, blockIdx.x, blockIdx.y, blockIdx.z - sl * zch, gridDim.x, gridDim.y);
 }
 __global__ void __launch_bounds__(NT) project_refine_kernel_b(const SlotArgs<float>* __restrict__ slots, int zch) {
   const int sl = blockIdx.z / zch;
@@ -1314,15 +1313,14 @@ template <class T> cudaError_t launch_momentum(const StencilArgs<T>& a, bool pf,
   return cudaGetLastError();
 }
 
-template <class T> cudaError_t launch_project(const StencilArgs<T>& a, cudaStream_t st) {
+cudaError_t launch_project(const StencilArgs<double>& a, cudaStream_t st) {
   const int n = a.c.n;
   dim3 grid(n / TX, n / TY, n / project_kz(n));
   switch (project_kz(n)) {
-    case 64: project_kernel<T, 64><<<grid, NT, 0, st>>>(a); break;
-    case 32: project_kernel<T, 32><<<grid, NT, 0, st>>>(a); break;
-    case 16: project_kernel<T, 16><<<grid, NT, 0, st>>>(a); break;
-    case 8: project_kernel<T, 8><<<grid, NT, 0, st>>>(a); break;
-    default: project_kernel<T, 4><<<grid, NT, 0, st>>>(a); break;
+    case 64: project_kernel<64><<<grid, NT, 0, st>>>(a); break;
+    case 16: project_kernel<16><<<grid, NT, 0, st>>>(a); break;
+    case 8: project_kernel<8><<<grid, NT, 0, st>>>(a); break;
+    default: project_kernel<4><<<grid, NT, 0, st>>>(a); break;
   }
   return cudaGetLastError();
 }
@@ -1383,11 +1381,10 @@ cudaError_t launch_project_batched(const SlotArgs<T>* slots, int nslots, int n, 
   dim3 grid(n / TX, n / TY, (n / project_kz(n)) * nslots);
   if constexpr (sizeof(T) == 8) {
     switch (project_kz(n)) {
-      case 64: project_kernel_b<T, 64><<<grid, NT, 0, st>>>(slots, n / project_kz(n)); break;
-      case 32: project_kernel_b<T, 32><<<grid, NT, 0, st>>>(slots, n / project_kz(n)); break;
-      case 16: project_kernel_b<T, 16><<<grid, NT, 0, st>>>(slots, n / project_kz(n)); break;
-      case 8: project_kernel_b<T, 8><<<grid, NT, 0, st>>>(slots, n / project_kz(n)); break;
-      default: project_kernel_b<T, 4><<<grid, NT, 0, st>>>(slots, n / project_kz(n)); break;
+      case 64: project_kernel_b<64><<<grid, NT, 0, st>>>(slots, n / project_kz(n)); break;
+      case 16: project_kernel_b<16><<<grid, NT, 0, st>>>(slots, n / project_kz(n)); break;
+      case 8: project_kernel_b<8><<<grid, NT, 0, st>>>(slots, n / project_kz(n)); break;
+      default: project_kernel_b<4><<<grid, NT, 0, st>>>(slots, n / project_kz(n)); break;
     }
   } else
     project_refine_kernel_b<<<grid, NT, 0, st>>>(slots, n / project_kz(n));
@@ -1404,8 +1401,6 @@ template cudaError_t launch_phase<double>(const StencilArgs<double>&, cudaStream
 template cudaError_t launch_phase<float>(const StencilArgs<float>&, cudaStream_t, int);
 template cudaError_t launch_momentum<double>(const StencilArgs<double>&, bool, cudaStream_t, int, int);
 template cudaError_t launch_momentum<float>(const StencilArgs<float>&, bool, cudaStream_t, int, int);
-template cudaError_t launch_project<double>(const StencilArgs<double>&, cudaStream_t);
-template cudaError_t launch_project<float>(const StencilArgs<float>&, cudaStream_t);
 template cudaError_t launch_materialize<double>(double*, double*, double*, int, Ctrl*, cudaStream_t);
 template cudaError_t launch_materialize<float>(float*, float*, float*, int, Ctrl*, cudaStream_t);
 
