@@ -15,9 +15,8 @@ namespace mhit {
 // because rounding is monotonic; then gamma, CFL, AB2 switch and the sticky
 // error status.  Partials hold STRIDE values per CTA: sums of u, v, w, maxima
 // of u, v, w, and (STRIDE 7, FP32 refine form) the max |div u| of the FP64
-// projection, which a NaN stays in.  The order of the sums depends on nparts
-// and NT only.  Not inlined: one CTA runs it, and the loop before it keeps its
-// own registers.
+// projection.  The order of the sums depends on nparts and NT only.  Not
+// inlined: one CTA runs it, and the loop before it keeps its own registers.
 template <int NT, int STRIDE>
 __device__ __noinline__ void finalize_step(const double* partials, int nparts, Ctrl* ctrl, double nd, double dt,
                                            double dxi) {
@@ -27,7 +26,7 @@ __device__ __noinline__ void finalize_step(const double* partials, int nparts, C
 #pragma unroll
     for (int t = 0; t < STRIDE; ++t) {
       const double x = __ldcg(partials + (size_t)b * STRIDE + t);
-      v[t] = t < 3 ? v[t] + x : (t < 6 ? fmax(v[t], x) : max_nan(v[t], x));
+      v[t] = t < 3 ? v[t] + x : fmax(v[t], x);
     }
   }
   __shared__ double red[NT / 32][7];
@@ -36,7 +35,7 @@ __device__ __noinline__ void finalize_step(const double* partials, int nparts, C
 #pragma unroll
     for (int t = 0; t < 7; ++t) {
       const double x = __shfl_xor_sync(0xffffffffu, v[t], o);
-      v[t] = t < 3 ? v[t] + x : (t < 6 ? fmax(v[t], x) : max_nan(v[t], x));
+      v[t] = t < 3 ? v[t] + x : fmax(v[t], x);
     }
   }
   if ((threadIdx.x & 31) == 0) {
@@ -47,10 +46,7 @@ __device__ __noinline__ void finalize_step(const double* partials, int nparts, C
   if (threadIdx.x == 0) {
     for (int w = 1; w < NT / 32; ++w) {
 #pragma unroll
-      for (int t = 0; t < 7; ++t)
-        red[0][t] = t < 3   ? red[0][t] + red[w][t]
-                    : t < 6 ? fmax(red[0][t], red[w][t])
-                            : max_nan(red[0][t], red[w][t]);
+      for (int t = 0; t < 7; ++t) red[0][t] = t < 3 ? red[0][t] + red[w][t] : fmax(red[0][t], red[w][t]);
     }
     const double um = red[0][0] / nd / nd / nd;
     const double vm = red[0][1] / nd / nd / nd;
@@ -68,9 +64,10 @@ __device__ __noinline__ void finalize_step(const double* partials, int nparts, C
     ctrl->cfl = cou;
     ctrl->alpha = 1.5;
     ctrl->beta = 0.5;
-    ctrl->max_div = (STRIDE > 6) ? red[0][6] : -1.0;
     ctrl->nstep += 1;
     const double s = red[0][0] + red[0][1] + red[0][2];
+    // the maximum drops a NaN, which the sums of the same velocities keep
+    ctrl->max_div = (STRIDE > 6) ? (s != s ? s : red[0][6]) : -1.0;
     if (!isfinite(s) || !isfinite(umax)) ctrl->status = 5;  // MHIT_ERR_NONFINITE
     else if (cou > ctrl->cfl_limit) ctrl->status = 4;      // MHIT_ERR_CFL
   }

@@ -1,6 +1,7 @@
 // Stencil kernels of the MHIT36 step on one B200: the ACDI phase-field update,
-// the momentum RHS + AB2 predictor, the projection with the mean/max
-// reductions, and the one-block finalize.
+// the momentum RHS + AB2 predictor, the unfused projections with the mean/max
+// reductions (FP32: and a one-CTA finalize), and the FP32 form's divergence
+// check.
 //
 // Fields are stored without halo cells, x fastest (n^3 values); periodic
 // neighbours come from index wrap.  On one rank this is exactly what the
@@ -29,11 +30,13 @@ constexpr int TX = 32, TY = 8, NT = TX * TY;
 // Default number of z chunks of a stencil kernel with `tiles` column tiles and
 // `slots` CTAs resident on the GPU.  Large grids: chunks of 32 planes, 64 from
 // 512^3 up (2-3% faster than 32 there; a chunk recomputes a few planes to
-// fill its rings).  A grid with less than two waves of such CTAs is split
-// further, to the number of chunks that gives the fewest iterations: an
-// iteration takes about the same time (2.4 us for FP64 phase) however many CTAs
-// share an SM, so waves * (longest chunk + lead) is what counts, lead being the
-// planes a chunk recomputes.  Chunks need not divide n evenly.
+// fill its rings).  A grid with less than two waves of such CTAs (up to 192^3,
+// and the FP32 phase kernel at 256^3, 182 us in 9 chunks against 190 in 8) is
+// split into the number of chunks, from n/32 up, with the least waves * (longest
+// chunk + lead), lead being the planes a chunk recomputes.  Chunks need not
+// divide n evenly.  The cost takes an iteration's time as the same however many
+// CTAs share an SM, which holds roughly only (FP64 phase: 2.4 us with one CTA
+// per SM at 32^3, 4.4 with three at 128^3).
 // B200, FP64 step against chunks of 32 planes everywhere (with project_kz):
 // 32^3 NS 108 -> 72 us a call, 64^3 182 -> 62 us a step, 128^3 277 -> 214,
 // 192^3 664 -> 627; chunks of 2 or 4 planes cost 128^3 30% and 256^3 30-80%.
@@ -816,14 +819,16 @@ __device__ __forceinline__ void momentum_body(const StencilArgs<T>& a, int nz, i
 // ============================================================ projection
 // C2 + R1 (multi/main.f90:873-903): u = ustar - dt/rho*(p - p_m)*dxi, with the
 // sums and maxima of the projected u, v, w reduced per CTA in FP64.
-// z planes per projection CTA: 64 (512^3: FP64 projection plus
+// z planes per projection CTA: 64 where n allows (512^3: FP64 projection plus
 // finalize 1.47 -> 1.41 ms against 16 planes, with a quarter of the partials
 // to reduce; FP32 projection 1.85 -> 1.49 ms); fewer on small grids, so that
 // they too fill the GPU (FP64: 32^3 21 -> 8 us, 64^3 42 -> 9 us, 96^3 25 -> 14
 // us, 128^3 68 -> 30 us, 192^3 92 -> 86 us).  The FP64 loop takes it as a
-// compile-time trip count (a run-time one measured 1.79 ms at 512^3).
+// compile-time trip count (a run-time one measured 1.79 ms at 512^3); the FP32
+// refinement's loop, with a run-time one, depends on how the compiler unrolls it
+// (384^3: 614 us as it stands, 644 not unrolled, 734 by 4 on request).
 __host__ __device__ constexpr int project_kz(int n) {
-  return n <= 96 ? 4 : (n <= 128 ? 8 : (n <= 192 ? 16 : 64));
+  return n <= 96 ? 4 : (n <= 128 ? 8 : (n <= 192 ? 16 : (n % 64 == 0 ? 64 : 32)));
 }
 
 template <int PKZ>
@@ -927,7 +932,8 @@ __device__ __forceinline__ void project_refine_body(const StencilArgs<float>& a,
     const double v1 = (double)a.vs[gyp] - dtr * (P(gyp) - pc) * dxi;
     const double w1 = wsn - dtr * (pn - pc) * dxi;
     const double div = ((u1 - uo) + (v1 - vo) + (w1 - wo)) * dxi;
-    mdiv = max_nan(mdiv, fabs(div));
+    mdiv = fmax(mdiv, fabs(div));
+    if (div != div) mdiv = NAN;
     a.uo[g] = (float)uo;
     a.vo[g] = (float)vo;
     a.wo[g] = (float)wo;
@@ -948,8 +954,7 @@ __device__ __forceinline__ void project_refine_body(const StencilArgs<float>& a,
 #pragma unroll
     for (int t = 0; t < 3; ++t) vals[t] += __shfl_xor_sync(0xffffffffu, vals[t], o);
 #pragma unroll
-    for (int t = 3; t < 6; ++t) vals[t] = fmax(vals[t], __shfl_xor_sync(0xffffffffu, vals[t], o));
-    vals[6] = max_nan(vals[6], __shfl_xor_sync(0xffffffffu, vals[6], o));
+    for (int t = 3; t < 7; ++t) vals[t] = fmax(vals[t], __shfl_xor_sync(0xffffffffu, vals[t], o));
   }
   __shared__ double red[NT / 32][7];
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
@@ -961,8 +966,7 @@ __device__ __forceinline__ void project_refine_body(const StencilArgs<float>& a,
     for (int t = 0; t < 7; ++t) r[t] = red[0][t];
     for (int w = 1; w < NT / 32; ++w) {
       for (int t = 0; t < 3; ++t) r[t] += red[w][t];
-      for (int t = 3; t < 6; ++t) r[t] = fmax(r[t], red[w][t]);
-      r[6] = max_nan(r[6], red[w][6]);
+      for (int t = 3; t < 7; ++t) r[t] = fmax(r[t], red[w][t]);
     }
     const size_t b = (size_t)bx + (size_t)gx * (by + (size_t)gy * bz);
     for (int t = 0; t < 7; ++t) a.partials[b * 7 + t] = r[t];
