@@ -56,13 +56,12 @@ ALGO_BYTES_STEP = {"fp64": {True: 280, False: 232}, "fp32": {True: 200, False: 1
 
 # DRAM bytes (read + write) per grid point per launch, from ncu captures of
 # the FP64 kernels at 256^3 (dram__bytes_read.sum + dram__bytes_write.sum of
-# a launch / 256^3; summaries in profiles/momentum_fp64_256_full.md,
-# profiles/phase_fp64_256_full.md and, for the Poisson kernels,
-# profiles/kernels_fp64_256_full.md).  A stencil or column pass touches every
-# point the same way at any size, so traffic scales with the points
-# processed; a full 512^3 capture is too large to take under ncu.
-DRAM_BYTES_PER_POINT_FP64 = {"momentum": 103.45, "phase": 40.25, "project": 54.13, "xfwd": 30.80,
-                             "yfwd": 13.59, "zsolve": 13.64, "yinv": 13.59, "xinv": 13.82, "xinvproj": 55.30}
+# a launch / 256^3; summary in profiles/kernels_fp64_256_full.md).  A stencil
+# or column pass touches every point the same way at any size, so traffic
+# scales with the points processed; a full 512^3 capture is too large to take
+# under ncu.
+DRAM_BYTES_PER_POINT_FP64 = {"momentum": 103.40, "phase": 41.43, "project": 54.13, "xfwd": 30.78,
+                             "yfwd": 13.68, "zsolve": 13.53, "yinv": 13.66, "xinv": 13.82, "xinvproj": 55.62}
 
 
 def kernel_bytes_per_point(n: int, pf: bool, precision: str = "fp64") -> dict:

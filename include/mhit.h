@@ -85,9 +85,9 @@ typedef struct mhit_diag {
   double cfl;      /* gumax*dt*dxi (multi/main.f90:942) */
   double umean, vmean, wmean; /* means removed by the step (multi/main.f90:906-919) */
   double gamma;    /* ACDI gamma used by the next step (1.0*gumax, multi/main.f90:362) */
-  double max_div;  /* FP32 refine form: max |div u| of the last step's FP64 projection (from 256^3 up
-                      measured when mhit_step / mhit_get_diag return, from the stored ustar, p0 and
-                      correction spectrum); -1 in the FP64 form */
+  double max_div;  /* FP32 refine form: max |div u| of the last step's FP64 projection (at 256^3,
+                      512^3 and 1024^3 measured when mhit_step / mhit_get_diag return, from the
+                      stored ustar, p0 and correction spectrum); -1 in the FP64 form */
   int64_t step;    /* steps taken since set_fields/load */
   int32_t status;  /* MHIT_OK or the sticky device error */
   int32_t reserved;
@@ -135,8 +135,8 @@ int mhit_set_fields(mhit_handle* h, const double* u, const double* v, const doub
  * Halo cells of MHIT_LAYOUT_PIX_HALO are filled periodically. */
 int mhit_get_fields(mhit_handle* h, double* u, double* v, double* w, double* phi, int layout);
 
-/* Download the last pressure p (multi/main.f90:842-850).  From 256^3 up the
- * FP64 step fuses the x inverse FFT into the projection and does not store
+/* Download the last pressure p (multi/main.f90:842-850).  At 256^3, 512^3
+ * and 1024^3 the FP64 step fuses the x inverse FFT into the projection and does not store
  * p; this call then recomputes it from the last step's spectrum (one x
  * inverse pass on the device) before the download.  The FP32 refinement form
  * returns p0 + dp, recomputing dp from the correction solve's spectrum the
