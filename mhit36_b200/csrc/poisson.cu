@@ -207,7 +207,9 @@ static size_t rcolsmem() {  // exchange buffer, twiddle table, prefetch buffer
   return (head + 127) / 128 * 128 + (size_t)R::E * R::NT * sizeof(typename C2<T>::t) + 8;
 }
 
-template <int N, int KIND, class T, bool PF, bool TMA, class Getter>
+// STOPS: the slabs belong to simulations that may have stopped; a stand-alone
+// solve's kernels (DEP) have no status to heed.
+template <int N, int KIND, class T, bool PF, bool TMA, bool STOPS, class Getter>
 __device__ __forceinline__ void rcol_run(int total, const typename C2<T>::t* __restrict__ gtw, Getter get) {
   typedef typename C2<T>::t C;
   constexpr int CC = RCfg<N, T>::CC, E = RCfg<N, T>::E, TPC = N / E;
@@ -225,6 +227,7 @@ __device__ __forceinline__ void rcol_run(int total, const typename C2<T>::t* __r
       mbar_init(bar, 1);
       mbar_init_fence();
     }
+    if constexpr (!STOPS) __syncthreads();
   }
   unsigned phase = 0;
   bool pend = false;  // a box load of the next slab is in flight (the same in every thread)
@@ -274,7 +277,7 @@ __device__ __forceinline__ void rcol_run(int total, const typename C2<T>::t* __r
   ColSlab nx;
   if constexpr (PF) {
     nx = get(blockIdx.x);
-    if constexpr (TMA) nx.live = agree(nx.live);  // also publishes the slot barrier
+    if constexpr (TMA && STOPS) nx.live = agree(nx.live);  // also publishes the slot barrier
     prefetch(nx);
   }
   for (int it = blockIdx.x; it < total; it += gridDim.x) {
@@ -297,7 +300,10 @@ __device__ __forceinline__ void rcol_run(int total, const typename C2<T>::t* __r
       }
       nx.live = false;
       if (it + (int)gridDim.x < total) nx = get(it + gridDim.x);
-      if constexpr (TMA) nx.live = agree(nx.live);  // every thread has read the buffer the next box fills
+      if constexpr (TMA) {  // every thread has read the buffer the next box fills
+        if constexpr (STOPS) nx.live = agree(nx.live);
+        else __syncthreads();
+      }
       prefetch(nx);
       if (!sl.live) continue;
     } else {
@@ -350,7 +356,7 @@ __global__ void __launch_bounds__(RCfg<N, T>::NT, RCfg<N, T>::minb(KIND)) rcol_k
   typedef PCfg<N, T> G;
   if (DEP) dep_begin();
   constexpr bool PFS = RCfg<N, T>::pf_single(KIND);
-  rcol_run<N, KIND, T, PFS, PFS>(G::NCHUNK * N, tw, [&](int it) {
+  rcol_run<N, KIND, T, PFS, PFS, !DEP>(G::NCHUNK * N, tw, [&](int it) {
     ColSlab s = slab_single<N, KIND, T>(spec, tw, k2tab, ctrl, it);
     s.map = &map;
     return s;
@@ -367,7 +373,7 @@ __global__ void __launch_bounds__(RCfg<N, T>::NT, RCfg<N, T>::minb(KIND)) rcol_k
     if (slots[q].active) tw = (which ? slots[q].pr : slots[q].po).tw;
   if (!tw) return;
   constexpr bool PFB = RCfg<N, T>::pf_batched(KIND);
-  rcol_run<N, KIND, T, PFB, PFB>(per * nslots, tw, [&](int it) {
+  rcol_run<N, KIND, T, PFB, PFB, true>(per * nslots, tw, [&](int it) {
     const int sl = it / per;
     const PoissonArgs<T>& a = which ? slots[sl].pr : slots[sl].po;
     ColSlab s;
